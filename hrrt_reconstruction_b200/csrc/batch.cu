@@ -142,24 +142,14 @@ int autotune(hrrt_ctx *ctx, const SubsetBufs &bb, int repeats, hrrt_tuning *chos
   }
   if (int rc = apply_tune(ctx, best)) return rc;
   if (!adj) {
-    for (int i = 0; i < 12; i++) {
-      ProjTune t = best;
-      t.bp_planes = (i & 1) ? 4 : 8;
-      t.bp_threads = (i & 2) ? 384 : 256;
-      t.bp_tile = (i < 4) ? 2 : (i < 8) ? 4 : 8;
-      double ms = 0;
-      int rc = time_launch(ctx, repeats, [&] {
-        return launch_bp(ctx->dg, bb.ratio, ctx->quad_pair, bw, ctx->bp_cnt[s], bb.bc, bb.br, ctx->vol, t, bb.fr,
-                         ctx->stream);
-      }, &ms);
-      if (rc) return rc;
-      if (ms < best_bp) {
-        best_bp = ms;
-        best.bp_planes = t.bp_planes;
-        best.bp_threads = t.bp_threads;
-        best.bp_tile = t.bp_tile;
-      }
-    }
+    // the back projector has one shape
+    int rc = time_launch(ctx, repeats, [&] {
+      return launch_bp(ctx->dg, bb.ratio, ctx->quad_pair, bw, ctx->bp_cnt[s], bb.bc, bb.br, ctx->vol, bb.fr,
+                       ctx->stream);
+    }, &best_bp);
+    if (rc) return rc;
+    best.bp_planes = 8;
+    best.bp_threads = 384;
   } else {
     best_bp = 0;
   }
@@ -276,7 +266,7 @@ int hrrt_get_tuning(hrrt_ctx *ctx, hrrt_tuning *t) {
   std::memset(t, 0, sizeof(*t));
   t->fp_planes = ctx->tune.fp_planes > 0 ? ctx->tune.fp_planes : kFpPlanes;
   t->fp_producer_warps = ctx->tune.fp_pwarps;
-  t->bp_planes = ctx->tune.bp_planes > 0 ? ctx->tune.bp_planes : kBpZ;
+  t->bp_planes = ctx->tune.bp_planes > 0 ? ctx->tune.bp_planes : 8;
   t->bp_threads = ctx->tune.bp_threads;
   t->bp_tile = ctx->tune.bp_tile;
   return HRRT_OK;

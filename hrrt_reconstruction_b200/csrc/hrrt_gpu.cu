@@ -241,7 +241,7 @@ int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
     } else {
       {
         Launch L(ctx, "bp_kernel");
-        CK(launch_bp(g, b.ratio, ctx->quad_pair, bw, ctx->bp_cnt[s], b.bc, b.br, ctx->vol, ctx->tune, b.fr,
+        CK(launch_bp(g, b.ratio, ctx->quad_pair, bw, ctx->bp_cnt[s], b.bc, b.br, ctx->vol, b.fr,
                      ctx->stream),
            "bp_kernel");
       }
@@ -279,7 +279,7 @@ int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
                            ctx->stream),
          "adj_rotate_kernel");
     } else {
-      CK(launch_bp(g, b.ratio, ctx->quad_pair, bw, ctx->bp_cnt[s], b.bc, b.br, ctx->vol, ctx->tune, b.fr,
+      CK(launch_bp(g, b.ratio, ctx->quad_pair, bw, ctx->bp_cnt[s], b.bc, b.br, ctx->vol, b.fr,
                    ctx->stream),
          "bp_kernel");
       CK(launch_rotback(g, pv, ctx->npairs, b.bc, b.br, ctx->vol, nullptr, nullptr, ctx->d_corr, 3, b.fr,
@@ -309,7 +309,7 @@ int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
   }
   {
     Launch L(ctx, "bp_kernel");
-    CK(launch_bp(g, b.ratio, ctx->quad_pair, bw, ctx->bp_cnt[s], b.bc, b.br, ctx->vol, ctx->tune, b.fr, ctx->stream),
+    CK(launch_bp(g, b.ratio, ctx->quad_pair, bw, ctx->bp_cnt[s], b.bc, b.br, ctx->vol, b.fr, ctx->stream),
        "bp_kernel");
   }
   Launch L(ctx, "rotback_kernel");
@@ -364,7 +364,7 @@ int sens_subset(hrrt_ctx *ctx, int s) {
          "adj_rotate_kernel");
     } else {
       CK(launch_bp(g, ctx->d_ratio, ctx->quad_pair, ctx->d_work + ctx->bp_off[s], ctx->bp_cnt[s], ctx->d_bc,
-                   ctx->d_br, ctx->vol, ctx->tune, one_frame(), ctx->stream),
+                   ctx->d_br, ctx->vol, one_frame(), ctx->stream),
          "bp_kernel");
       CK(launch_rotback(g, pv, ctx->npairs, ctx->d_bc, ctx->d_br, ctx->vol, nullptr, nullptr, ctx->d_corr, 3,
                         one_frame(), ctx->stream),
@@ -397,7 +397,7 @@ int sens_subset(hrrt_ctx *ctx, int s) {
   {
     Launch L(ctx, "bp_kernel");
     CK(launch_bp(ctx->dg, ctx->d_ratio, ctx->quad_pair, ctx->d_work + ctx->bp_off[s], ctx->bp_cnt[s], ctx->d_bc,
-                 ctx->d_br, ctx->vol, ctx->tune, one_frame(), ctx->stream),
+                 ctx->d_br, ctx->vol, one_frame(), ctx->stream),
        "bp_kernel");
   }
   Launch L(ctx, "rotback_kernel");
@@ -624,18 +624,23 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
   std::vector<int16_t> plane_seg(g.segmentsize);
   for (int s = 0; s < g.nseg; s++)
     for (int r = 0; r <= g.yr_top[s] - g.yr_bottom[s]; r++) plane_seg[g.segment_offset[s] + r] = (int16_t)s;
-  // back-projection shared-memory layout: every segment with kBpPad zero
-  // planes on each side; bp_src[i] = quad-layout plane of shared plane i or -1
+  // back-projection shared-memory layout: kBpPad zero planes before, between
+  // and after the segments, plane yr of a segment at a position = yr modulo 4;
+  // bp_src[i] = quad-layout plane of shared plane i or -1
   std::vector<int> bp_soff(g.nseg), bp_src;
+  size_t bp_padded = 0;  // with kBpPad planes on both sides of every segment
   for (int s = 0; s < g.nseg; s++) {
     const int ns = g.yr_top[s] - g.yr_bottom[s] + 1;
-    for (int k = 0; k < kBpPad; k++) bp_src.push_back(-1);
+    for (int k = 0; k < kBpPad || ((int)bp_src.size() - g.yr_bottom[s]) % 4 != 0; k++) bp_src.push_back(-1);
     bp_soff[s] = (int)bp_src.size();
     for (int r = 0; r < ns; r++) bp_src.push_back(g.padded_offset(s) + r);
-    for (int k = 0; k < kBpPad; k++) bp_src.push_back(-1);
+    bp_padded += ns + 2 * kBpPad;
   }
-  // whole groups of 8 planes: the back projector swizzles within them
-  while (bp_src.size() % 8) bp_src.push_back(-1);
+  for (int k = 0; k < kBpPad; k++) bp_src.push_back(-1);
+  // slots per phase: 2 modulo 8, so that eight consecutive planes fall in
+  // different bank groups
+  int bp_s4 = ((int)bp_src.size() + 3) / 4;
+  while (bp_s4 % 8 != 2) bp_s4++;
   // no back-projection window may run past its segment's zero planes
   for (int y = 1; y < g.ny; y++)
     for (int gg = 0; gg < g.groupmax; gg++) {
@@ -643,9 +648,46 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
       const int zs = g.bl_zsa[i], ze = g.bl_zea[i], d = g.bl_yra[i] - g.bl_zsa[i];
       const int yb = g.yr_bottom[2 * gg + 2], yt = g.yr_top[2 * gg + 2];
       if (ze < zs) return bail(fail(ctx, HRRT_ERR_ARG, "bp: empty plane range"));
-      const int z_lo = (zs / kBpZ) * kBpZ, z_hi = (ze / kBpZ) * kBpZ + kBpZ - 1;
+      const int z_lo = (zs / kAdjZ) * kAdjZ, z_hi = (ze / kAdjZ) * kAdjZ + kAdjZ - 1;
       if (z_lo + d < yb - kBpPad || z_hi + d + 1 > yt + kBpPad) return bail(fail(ctx, HRRT_ERR_ARG, "bp: padding"));
     }
+  // the back projector's row groups: per (group, side) the rows kBpRows*m .. +3
+  // (side 1: their mirrors ny - y); rows outside 1..c take the nearest one's
+  // entry and are not stored
+  const int bpm = g.c / kBpRows + 1;
+  std::vector<BpRows> bprows((size_t)g.groupmax * 2 * bpm);
+  for (int gg = 0; gg < g.groupmax; gg++)
+    for (int side = 0; side < 2; side++)
+      for (int m = 0; m < bpm; m++) {
+        BpLut l[kBpRows];
+        for (int r = 0; r < kBpRows; r++) {
+          const int y = std::min(std::max(kBpRows * m + r, 1), g.c);
+          l[r] = bpl[(size_t)gg * g.ny + (side ? g.ny - y : y)];
+        }
+        const size_t at = ((size_t)m * g.groupmax + gg) * 2 + side;
+        int lo = l[0].d, hi = l[0].d, zs = l[0].zs, ze = l[0].ze;
+        for (const BpLut &b : l) {
+          lo = std::min(lo, b.d);
+          hi = std::max(hi, b.d);
+          zs = std::min(zs, b.zs);
+          ze = std::max(ze, b.ze);
+        }
+        BpRows &e = bprows[at];
+        for (int k = 0; k < 4; k++) e.off[k] = (int16_t)(((lo + k) & 3) * bp_s4 + ((lo + k) >> 2));
+        e.zs = (int16_t)zs;
+        e.ze = (int16_t)ze;
+        e.k = 0;
+        for (int r = 0; r < kBpRows; r++) {
+          e.u[r] = l[r].d > lo ? l[r].f : l[r].f - 1.0f;
+          e.k += l[r].d > lo;
+        }
+        bool wide = hi - lo > 1;
+        for (int r = 0; r < kBpRows; r++) wide = wide || (l[r].d > lo) != (side ? r >= kBpRows - e.k : r < e.k);
+        // no window of a run that meets [zs, ze] may leave the segment's zero planes
+        const int yb = g.yr_bottom[2 * gg + 2], yt = g.yr_top[2 * gg + 2];
+        const int z_lo = (zs / kBpZ) * kBpZ, z_hi = (ze / kBpZ) * kBpZ + kBpZ - 1;
+        if (wide || z_lo + lo < yb - kBpPad || z_hi + lo + 2 > yt + kBpPad) e.k = kBpWide;
+      }
   // forward-projection task lists of every plane variant (one task per
   // consumer thread, two producer warps at least); the default variant must
   // fit, the others are offered to the tuner where they do
@@ -663,10 +705,10 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
   if (!m.empty()) return bail(fail(ctx, HRRT_ERR_ARG, m));
   if (g.groupmax > kFpMaxGroups)
     return bail(fail(ctx, HRRT_ERR_ARG, "fp: more segment groups than the projector stages per row"));
-  if (g.zp % kBpZ != 0) return bail(fail(ctx, HRRT_ERR_ARG, "padded z must be a multiple of 8"));
+  if (g.zp % kAdjZ != 0) return bail(fail(ctx, HRRT_ERR_ARG, "padded z must be a multiple of 8"));
   for (int x = 1; x <= g.c; x++)
     if (g.cyl0[x] != g.cyl1[x] && g.cyl0[x] < 1) return bail(fail(ctx, HRRT_ERR_ARG, "FOV reaches the grid edge"));
-  if ((size_t)bp_src.size() * 16 > 200 * 1024)
+  if ((bp_padded + 7) / 8 * 8 * 16 > 200 * 1024)
     return bail(fail(ctx, HRRT_ERR_ARG, "sinogram quad exceeds shared memory"));
 
   DevGeom &d = ctx->dg;
@@ -739,6 +781,7 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
     d.adj_cnt = d.adj_ent ? dalloc<int>(ctx, (size_t)ctx->npairs * g.nx * g.nx, &e) : nullptr;
   }
   d.bplut = dupload(ctx, bpl, &e);
+  d.bprows = dupload(ctx, bprows, &e);
   d.sin_psi = dupload(ctx, g.sin_psi, &e);
   d.cos_psi = dupload(ctx, g.cos_psi, &e);
   d.fov_xy = dupload(ctx, fovxy, &e);
@@ -759,6 +802,7 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
   d.bp_soff = dupload(ctx, bp_soff, &e);
   d.bp_src = dupload(ctx, bp_src, &e);
   d.bp_splanes = (int)bp_src.size();
+  d.bp_s4 = bp_s4;
   ctx->d_rowstart = dupload(ctx, rowstart, &e);
   d.err = dalloc<int>(ctx, 1, &e);
   d.range_err = dalloc<int>(ctx, 1, &e);
@@ -1420,7 +1464,7 @@ int hrrt_bp_pair(hrrt_ctx *ctx, const float *prj, int view, float *imagebuf_xyz,
   CK(launch_rows_to_quad(ctx->dg, g.nbins, ctx->d_rows, ctx->d_ratio, 1, ctx->stream), "pack");
   {
     Launch L(ctx, "bp_kernel");
-    CK(launch_bp(ctx->dg, ctx->d_ratio, ctx->quad_pair, dw, (int)work.size(), ctx->d_bc, ctx->d_br, ctx->vol, ctx->tune, one_frame(),
+    CK(launch_bp(ctx->dg, ctx->d_ratio, ctx->quad_pair, dw, (int)work.size(), ctx->d_bc, ctx->d_br, ctx->vol, one_frame(),
                  ctx->stream),
        "bp_kernel");
   }

@@ -8,6 +8,7 @@
 
 #include <cuda.h>  // CUtensorMap (the encoder is reached through the runtime's driver entry point)
 
+#include <algorithm>
 #include <cfloat>
 #include <cstring>
 #include <type_traits>
@@ -564,45 +565,84 @@ __global__ void __launch_bounds__(MW * 32, 1) fp_kernel(DevGeom g, const float *
 }
 
 // ============================================================================
-// Back projection, one CTA per (view pair, quad x).  Voxel-driven restatement
-// of back_proj3d_view_n1thread (sbrt:4162-4668): the quad's four sinogram
-// lanes sit in shared memory; each thread evaluates, for its rotated-grid row
-// y and a run of kBpZ planes, the two 4-lane sums the reference builds
-// incrementally (sumt1 for voxels (x,y),(N-x,y),(N-y,x),(N-y,N-x); sumt2 for
-// (x,N-y),(N-x,N-y),(y,x),(y,N-x)) as direct linear interpolations of the
-// zero-padded sinogram at yr = z + d.  Each voxel receives two partial sums,
-// one from the ray of view p (its column quad) and one from the ray of view
-// p+nviews/2 (its row quad); they go to Bc and Br and are added in the
-// rotate-back, which is the reference's assign-then-accumulate order.
+// Back projection, one CTA (or `split` CTAs) per (view pair, quad x).
+// Voxel-driven restatement of back_proj3d_view_n1thread (sbrt:4162-4668): the
+// quad's four sinogram lanes sit in shared memory; each thread evaluates, for
+// kBpRows rotated-grid rows y and a run of kBpZ planes, the two 4-lane sums the
+// reference builds incrementally (sumt1 for voxels (x,y),(N-x,y),(N-y,x),
+// (N-y,N-x); sumt2 for (x,N-y),(N-x,N-y),(y,x),(y,N-x)) as direct linear
+// interpolations of the zero-padded sinogram at yr = z + d.  Each voxel
+// receives two partial sums, one from the ray of view p (its column quad) and
+// one from the ray of view p+nviews/2 (its row quad); they go to Bc and Br and
+// are added in the rotate-back, which is the reference's assign-then-
+// accumulate order.
+// What bounds it is instruction issue and the latency that 14 warps leave
+// uncovered (FMA pipe about 40 % busy, L1 45 %): per (row group, side of a
+// group) a thread reads 6 shared planes for 16 outputs -- adjacent rows read
+// the segment less than a plane apart, so four rows share a window -- and
+// issues 50 packed FMAs and about 65 other instructions.  One row and 8
+// planes a thread (9 shared planes for 8 outputs, an address each) took
+// 1.384 ms a span-3 subset and 0.509 ms a span-9 one; this 0.892 and 0.361.
+// Measured and not used: the row pattern as arithmetic instead of a branch (both
+// slopes applied, one of them 0: 1.021 ms), lane pairs split over two threads
+// for twice the warps (0.941 ms), no prefetch of the next entry (0.977 ms).
 // ============================================================================
-// The shared planes are stored swizzled: plane i at bsw(i), its position
-// within its aligned group of 8 XORed with the group's index.  Threads of a
-// warp take consecutive 8-plane runs of one row, so their loads of the same
-// window offset are 8 planes (128 bytes) apart; the swizzle puts them in
-// different 16-byte bank groups without the shared memory a padding would
-// cost.
-__device__ __forceinline__ int bsw(int i) { return i ^ ((i >> 3) & 7); }
+// The shared planes are stored by phase, plane i at slot bp_slot(i): eight
+// lanes of a warp take consecutive 4-plane runs of one row group, so that
+// their loads of the same window offset are of one phase and contiguous.  The
+// segments sit at offsets that keep a plane's phase (context creation), so
+// the slots of a window's first four planes come from the row group's table
+// entry, and the next two are one slot after the first two.
+__device__ __forceinline__ int bp_slot(int i, int s4) { return (i & 3) * s4 + (i >> 2); }
+// the shared plane at a byte address
+__device__ __forceinline__ Q2 ldb(const float4 *P, int at) {
+  return ldq(reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(P) + at));
+}
 
+// one row of a wide entry on its own (steep segments of short scanners)
 template <int KB>
-__device__ __forceinline__ void bp_lerp(Q2 (&s)[KB], const float4 *__restrict__ P, int pbase, const BpLut &bl,
+__device__ __forceinline__ void bp_lerp(Q2 (&s)[KB], const float4 *__restrict__ P, int s4, int pbase, const BpLut &bl,
                                         int z0) {
   // windows wholly outside [zs, ze] contribute nothing; a window that
   // straddles an end reads the segment's zero planes for its outside planes
   if (z0 + KB - 1 < bl.zs || z0 > bl.ze) return;
   const int i0 = pbase + z0 + bl.d;
-  // the reference's p[yr] + f*(p[yr+1]-p[yr]) (sbrt:4312-4315) as
-  // (1-f) p[yr] + f p[yr+1], added with two fused multiply-adds
   const uint64_t f = pk(bl.f, bl.f), g = pk(1.0f - bl.f, 1.0f - bl.f);
-  Q2 a = ldq(P + bsw(i0));
+  Q2 a = ldq(P + bp_slot(i0, s4));
 #pragma unroll
   for (int j = 0; j < KB; j++) {
-    const Q2 b = ldq(P + bsw(i0 + j + 1));
+    const Q2 b = ldq(P + bp_slot(i0 + j + 1, s4));
     s[j] = qfma(b, f, qfma(a, g, s[j]));
     a = b;
   }
 }
 
-template <int KB, bool ACC = false>
+// one side of a segment group for a row group and a run of planes (BpRows):
+// the first (SIDE 0) or last (SIDE 1) K rows are one plane further on; A[k]
+// is where plane k of the window lies, A[0] + 16 and A[1] + 16 the next two.
+// The differences are fused multiply-adds by a run-time (-1, -1): a packed
+// subtraction costs two more instructions for the signs.
+template <int SIDE, int K>
+__device__ __forceinline__ void bp_rows(Q2 (&s)[kBpRows][kBpZ], Q2 (&com)[kBpZ], const float4 *__restrict__ P,
+                                        const int (&A)[4], const float4 &v, uint64_t neg1) {
+  const uint64_t u[kBpRows] = {pk(v.x, v.x), pk(v.y, v.y), pk(v.z, v.z), pk(v.w, v.w)};
+  Q2 w1 = ldb(P, A[1]), d0 = qfma(ldb(P, A[0]), neg1, w1);
+#pragma unroll
+  for (int j = 0; j < kBpZ; j++) {
+    com[j] = qadd(com[j], w1);
+    Q2 d1 = d0;
+    if (K > 0 || j + 1 < kBpZ) {
+      const Q2 w2 = ldb(P, j == 0 ? A[2] : j == 1 ? A[3] : j == 2 ? A[0] + 16 : A[1] + 16);
+      d1 = qfma(w1, neg1, w2);
+      w1 = w2;
+    }
+#pragma unroll
+    for (int r = 0; r < kBpRows; r++) s[r][j] = qfma((SIDE ? r >= kBpRows - K : r < K) ? d1 : d0, u[r], s[r][j]);
+    d0 = d1;
+  }
+}
+
+template <int KB>
 __device__ __forceinline__ void store_lane(float *__restrict__ dst, const Q2 (&s)[KB], int l) {
   float v[KB];
 #pragma unroll
@@ -610,10 +650,7 @@ __device__ __forceinline__ void store_lane(float *__restrict__ dst, const Q2 (&s
     const float2 t = upk(l < 2 ? s[j].lo : s[j].hi);
     v[j] = (l & 1) ? t.y : t.x;
   }
-  if (ACC) {
-#pragma unroll
-    for (int j = 0; j < KB; j++) atomicAdd(dst + j, v[j]);
-  } else if constexpr (KB == 8) {
+  if constexpr (KB == 8) {
     // one 32-byte store (sm_100): a whole sector per lane, one line touched
     // per row of the warp's task tile instead of two stores to each
     asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]),
@@ -625,119 +662,158 @@ __device__ __forceinline__ void store_lane(float *__restrict__ dst, const Q2 (&s
       *reinterpret_cast<float4 *>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
   }
 }
+// one lane of a run: stored, or (ACC) added to what is there by one 16-byte
+// reduction (sm_90+) where the caller's buffer is aligned for it
+template <bool ACC>
+__device__ __forceinline__ void put(float *__restrict__ dst, const Q2 (&s)[kBpZ], int l, bool vec) {
+  if constexpr (!ACC) {
+    store_lane<kBpZ>(dst, s, l);
+  } else {
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float2 t = upk(l < 2 ? s[j].lo : s[j].hi);
+      v[j] = (l & 1) ? t.y : t.x;
+    }
+    if (vec) {
+      asm volatile("red.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+                   : "memory");
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++) atomicAdd(dst + j, v[j]);
+    }
+  }
+}
 
-template <int KB, bool ACC = false, bool MULTI = false, int NT = 256>
-__global__ void __launch_bounds__(NT, NT >= 384 ? 2 : kBpMinBlocks) bp_kernel(DevGeom g, const float4 *__restrict__ in, long long in_pair_stride,
-                                                 const QuadWork *__restrict__ work, float *__restrict__ bc,
-                                                 float *__restrict__ br, long long vol, FrameStrides fr,
-                                                 int view0, int x0, int rlog) {
+// Two CTAs per SM (their shared planes fill it at span 3) of at most 128
+// registers a thread.  Measured on B200 (span 3 / span 9 subset): 192 threads
+// of 160 registers 941 / 368 us, 224 threads 892 / 361 us, 256 threads
+// 952 / 381 us; one view pair with ACC: 152, 169 and 142 us.
+template <bool ACC>
+constexpr int kBpThreads = ACC ? 256 : 224;
+
+template <bool ACC, bool MULTI>
+__global__ void __launch_bounds__(kBpThreads<ACC>, 2) bp_kernel(DevGeom g, const float4 *__restrict__ in,
+                                                           long long in_pair_stride, const QuadWork *__restrict__ work,
+                                                           float *__restrict__ bc, float *__restrict__ br,
+                                                           long long vol, FrameStrides fr, int view0, int x0,
+                                                           int split) {
+  constexpr int KB = kBpZ, KR = kBpRows, NT = kBpThreads<ACC>;
   extern __shared__ float4 P[];  // [bp_splanes]: segments with kBpPad zero planes each side
-  // ACC: one view pair, quads x0 + blockIdx.x, both partial sums added into bc
-  // (each voxel receives exactly two terms, so the atomic adds onto a zeroed
-  // buffer give a + b whatever their order)
-  // MULTI: several frames per launch (one frame: the frame arithmetic is
-  // compiled out, which keeps the single-frame kernel free of spills)
-  int item = blockIdx.x;
+  __shared__ int2 s_base[kFpMaxGroups];  // per group: byte offset of yr 0 of its even / odd segment (of its slot)
+  // ACC: one view pair, quads x0.., both partial sums added into bc (each
+  // voxel receives exactly two terms, so the atomic adds onto a zeroed buffer
+  // give a + b whatever their order)
+  // MULTI: several frames per launch
+  int item = blockIdx.x / split;
+  const int part = blockIdx.x - item * split;
   if (MULTI) {
-    const int nwork = gridDim.x / fr.n, frame = blockIdx.x / nwork;
-    item = blockIdx.x - frame * nwork;
+    const int nwork = gridDim.x / split / fr.n, frame = item / nwork;
+    item -= frame * nwork;
     in += (size_t)frame * fr.ratio / 4;
     bc += (size_t)frame * fr.bc;
     br += (size_t)frame * fr.bc;
   }
-  const QuadWork w = ACC ? QuadWork{0, (int16_t)(x0 + blockIdx.x), (int16_t)view0, 0} : work[item];
-  const int x = w.x, N = g.nx, c = g.c, zp = g.zp, G = g.groupmax;
+  const QuadWork w = ACC ? QuadWork{0, (int16_t)(x0 + item), (int16_t)view0, 0} : work[item];
+  const int x = w.x, N = g.nx, c = g.c, zp = g.zp, G = g.groupmax, s4 = g.bp_s4;
   const bool masked = g.nzmask[w.view * g.nquads + x] == 0;
   const float4 *src = in + (size_t)w.slot * in_pair_stride + (size_t)x * g.pplanes;
-  if (!masked)
-    for (int i = threadIdx.x; i < g.bp_splanes; i += blockDim.x) {
+  if (!masked) {
+#pragma unroll 8
+    for (int i = threadIdx.x; i < g.bp_splanes; i += NT) {
       const int q = __ldg(g.bp_src + i);
-      P[bsw(i)] = (q >= 0) ? src[q] : f4(0.f);
+      P[bp_slot(i, s4)] = (q >= 0) ? __ldg(src + q) : f4(0.f);
     }
+    if (threadIdx.x < G)
+      s_base[threadIdx.x] = make_int2(4 * (g.bp_soff[2 * threadIdx.x + 2] - g.ybot[2 * threadIdx.x + 2]),
+                                      4 * (g.bp_soff[2 * threadIdx.x + 1] - g.ybot[2 * threadIdx.x + 2]));
+  }
   __syncthreads();
 
   // ACC: both partial sums go through bc (br is unused and may be null), so
   // the two destinations derive from one restrict pointer
   float *bcp = bc + (size_t)w.slot * vol;
   float *brp = (ACC ? bc : br) + (size_t)w.slot * vol;
-  const int ystart = g.cyl0[x];
-  const int nyq = c - ystart + 1, nzc = zp / KB;
-  const int o0 = g.bp_soff[0];
-  // task = (half, row, plane run); half 0 builds sumt1 (voxels (x,y),(N-x,y),
-  // (N-y,x),(N-y,N-x)), half 1 sumt2 (voxels (x,N-y),(N-x,N-y),(y,x),(y,N-x)).
-  // A warp's 32 tasks are a tile of R = 2^rlog consecutive plane runs of
-  // 32/R consecutive rows.  Along the runs a warp's stores of a voxel column
-  // are contiguous, and the swizzle spreads its shared loads over the banks;
-  // along the rows the row entries differ, but windows at the same planes
-  // and a slowly varying offset d(y) often coincide (broadcast).  Many
-  // segment groups favour few runs, few groups (store-heavy) many.
-  const int R = 1 << rlog, RW = 32 >> rlog;
-  const int CT = (nzc + R - 1) >> rlog, RT = (nyq + RW - 1) / RW;
-  const int per_half = RT * CT * 32;
-  for (int task = threadIdx.x; task < 2 * per_half; task += blockDim.x) {
-    const int half = task >= per_half;
-    const int t2 = task - half * per_half;
-    const int tile = t2 >> 5, l = t2 & 31, ty = tile / CT, tc = tile - ty * CT;
-    const int yi = ty * RW + (l >> rlog), zc = (tc << rlog) + (l & (R - 1)), z0 = zc * KB;
-    if (yi >= nyq || zc >= nzc) continue;
-    const int y = ystart + yi;
-    if (half && y == c) continue;  // the centre row has a single voxel set
-    Q2 s[KB];
-    if (masked) {
-      // masked quads contribute zero (sbrt:4223-4258, :4595-4640)
+  const bool vec = ACC && (reinterpret_cast<uintptr_t>(bc) & 15) == 0;
+  const uint64_t neg1 = pk(-g.unit, -g.unit);
+  const int ystart = g.cyl0[x], o0 = g.bp_soff[0];
+  const int m0 = ystart / KR, M = c / KR + 1, nm = M - m0, nzc = zp / KB;
+  // A warp takes 16 consecutive plane runs of one row group in both halves:
+  // half 0 builds sumt1, half 1 sumt2 (the centre row, y = c, has a single
+  // voxel set: half 0's).  The halves read the two segments of a group at the
+  // same position, so a warp's lanes take the same path through bp_rows.
+  const int lane = threadIdx.x & 31, half = lane >> 4;
+  const int CT = (nzc + 15) / 16, tiles = nm * CT;
+  const int step = split * (NT / 32);
+  for (int tile = part * (NT / 32) + (threadIdx.x >> 5); tile < tiles; tile += step) {
+    const int ty = tile / CT, tc = tile - ty * CT;
+    const int m = m0 + ty, zc = tc * 16 + (lane & 15), z0 = zc * KB;
+    if (zc >= nzc) continue;
+    Q2 s[KR][KB], com[KB];
 #pragma unroll
-      for (int j = 0; j < KB; j++) s[j] = Q2{0ull, 0ull};
-    } else if (y == c) {
-      // centre row (sbrt:4260-4284): rays pass plane yr = z exactly
+    for (int j = 0; j < KB; j++) {
+      com[j] = Q2{0ull, 0ull};
 #pragma unroll
-      for (int j = 0; j < KB; j++) s[j] = ldq(P + bsw(o0 + z0 + j));
-      for (int gg = 0; gg < G; gg++) {
-        const int se = 2 * gg + 2, so = 2 * gg + 1;
-        const int yb = g.ybot[se], yt = g.ytop[se];
-        const int pe = g.bp_soff[se] - yb, po = g.bp_soff[so] - yb;
+      for (int r = 0; r < KR; r++) s[r][j] = Q2{0ull, 0ull};
+    }
+    // masked quads contribute zero (sbrt:4223-4258, :4595-4640)
+    if (!masked) {
 #pragma unroll
-        for (int j = 0; j < KB; j++) {
-          const int z = z0 + j;
-          if (z >= yb && z <= yt) s[j] = qadd(s[j], qadd(ldq(P + bsw(pe + z)), ldq(P + bsw(po + z))));
+      for (int j = 0; j < KB; j++) com[j] = ldq(P + o0 / 4 + zc + j * s4);
+      const int4 *e = reinterpret_cast<const int4 *>(g.bprows + (size_t)m * G * 2);
+      int4 hn = __ldg(e);
+      float4 un = __ldg(reinterpret_cast<const float4 *>(e + 1));
+      // one side of group gg; sumt1: segment 2k at +u (side 0, rows y) and
+      // 2k-1 at -u (side 1, rows N-y); sumt2: the converse
+      auto side_of = [&](auto side_c, int gg, int seg, bool last) {
+        constexpr int SIDE = decltype(side_c)::value;
+        const int4 h = hn;
+        const float4 v = un;
+        if (!last) {  // the next entry, in flight under this one's planes
+          e += 2;
+          hn = __ldg(e);
+          un = __ldg(reinterpret_cast<const float4 *>(e + 1));
         }
-      }
-    } else {
+        if (z0 + KB - 1 < (int)(int16_t)(h.z & 0xffff) || z0 > (h.z >> 16)) return;
+        const int B = seg + 16 * zc;
+        const int A[4] = {B + 16 * (int)(int16_t)(h.x & 0xffff), B + 16 * (h.x >> 16),
+                          B + 16 * (int)(int16_t)(h.y & 0xffff), B + 16 * (h.y >> 16)};
+        switch (h.w) {
+          case 0: bp_rows<SIDE, 0>(s, com, P, A, v, neg1); break;
+          case 1: bp_rows<SIDE, 1>(s, com, P, A, v, neg1); break;
+          case 2: bp_rows<SIDE, 2>(s, com, P, A, v, neg1); break;
+          case 3: bp_rows<SIDE, 3>(s, com, P, A, v, neg1); break;
+          default:
 #pragma unroll
-      for (int j = 0; j < KB; j++) s[j] = ldq(P + bsw(o0 + z0 + j));
-      // bplut is [group][row]: the threads of a row read the same entries
-      const BpLut *l1 = g.bplut + y, *l2 = g.bplut + (N - y);
-      BpLut b1 = l1[0], b2 = l2[0];
+            for (int r = 0; r < KR; r++) {
+              const int y = min(max(KR * m + r, 1), c);
+              bp_lerp<KB>(s[r], P, s4, seg / 4, g.bplut[(size_t)gg * N + (SIDE ? N - y : y)], z0);
+            }
+        }
+      };
       for (int gg = 0; gg < G; gg++) {
-        const int se = 2 * gg + 2, so = 2 * gg + 1;
-        const int yb = g.ybot[se];
-        const int pe = g.bp_soff[se] - yb, po = g.bp_soff[so] - yb;
-        const int gn = (gg + 1 < G) ? gg + 1 : gg;
-        const BpLut n1 = l1[(size_t)gn * N], n2 = l2[(size_t)gn * N];  // next group, in flight
-        // sumt1: segment 2k at +u and 2k-1 at -u; sumt2: the converse
-        bp_lerp<KB>(s, P, half ? po : pe, b1, z0);
-        bp_lerp<KB>(s, P, half ? pe : po, b2, z0);
-        b1 = n1;
-        b2 = n2;
+        const int2 base = s_base[gg];
+        side_of(std::integral_constant<int, 0>{}, gg, half ? base.y : base.x, false);
+        side_of(std::integral_constant<int, 1>{}, gg, half ? base.x : base.y, gg + 1 == G);
       }
     }
-    // the reference writes planes z < nz only
 #pragma unroll
-    for (int j = 0; j < KB; j++)
-      if (z0 + j >= g.nz) s[j] = Q2{0ull, 0ull};
-    const size_t cz = (size_t)z0;
-    if (!half) {
-      store_lane<KB, ACC>(bcp + ((size_t)x * N + y) * zp + cz, s, 0);
-      store_lane<KB, ACC>(brp + ((size_t)(N - y) * N + x) * zp + cz, s, 2);
-      if (x != c) {
-        store_lane<KB, ACC>(bcp + ((size_t)(N - x) * N + y) * zp + cz, s, 1);
-        store_lane<KB, ACC>(brp + ((size_t)(N - y) * N + N - x) * zp + cz, s, 3);
+    for (int r = 0; r < KR; r++) {
+      const int y = KR * m + r;
+      if (y < ystart || y > c || (half && y == c)) continue;
+#pragma unroll
+      for (int j = 0; j < KB; j++) {
+        // the reference writes planes z < nz only
+        s[r][j] = qadd(s[r][j], com[j]);
+        if (z0 + j >= g.nz) s[r][j] = Q2{0ull, 0ull};
       }
-    } else {
-      store_lane<KB, ACC>(bcp + ((size_t)x * N + N - y) * zp + cz, s, 0);
-      store_lane<KB, ACC>(brp + ((size_t)y * N + x) * zp + cz, s, 2);
+      // column voxels (x, yc), (N-x, yc); row voxels (yr, x), (yr, N-x)
+      const int yc = half ? N - y : y, yr = half ? y : N - y;
+      put<ACC>(bcp + ((size_t)x * N + yc) * zp + z0, s[r], 0, vec);
+      put<ACC>(brp + ((size_t)yr * N + x) * zp + z0, s[r], 2, vec);
       if (x != c) {
-        store_lane<KB, ACC>(bcp + ((size_t)(N - x) * N + N - y) * zp + cz, s, 1);
-        store_lane<KB, ACC>(brp + ((size_t)y * N + N - x) * zp + cz, s, 3);
+        put<ACC>(bcp + ((size_t)(N - x) * N + yc) * zp + z0, s[r], 1, vec);
+        put<ACC>(brp + ((size_t)yr * N + N - x) * zp + z0, s[r], 3, vec);
       }
     }
   }
@@ -1452,54 +1528,36 @@ cudaError_t launch_fp(const DevGeom &g, const float *image, const QuadWork *work
   }
 }
 
-// log2 of the back projector's tile width (bp_kernel): the tuned one, else
-// 2 runs where there are many segment groups and 4 where there are few
-// (measured on B200 over 1..32: span 3 1.56 ms at 2, span 9 0.57 ms at 4);
-// -1 if invalid
-int bp_tile_log2(const DevGeom &g, const ProjTune &t) {
-  const int r = t.bp_tile > 0 ? t.bp_tile : (g.groupmax > 12 ? 2 : 4);
-  for (int l = 0; l <= 5; l++)
-    if (r == 1 << l) return l;
-  return -1;
-}
-
-template <int KB, int NT>
-cudaError_t launch_bp_t(const DevGeom &g, const float *in, long long in_pair_stride, const QuadWork *work, int nwork,
-                        float *bc, float *br, long long vol, const FrameStrides &fr, int rlog, cudaStream_t st) {
-  static_assert(kBpPad >= KB, "a straddling window must stay inside the zero planes");
-  const size_t smem = (size_t)g.bp_splanes * sizeof(float4);
-  auto k = fr.n > 1 ? bp_kernel<KB, false, true, NT> : bp_kernel<KB, false, false, NT>;
+template <bool ACC, bool MULTI>
+cudaError_t launch_bp_t(const DevGeom &g, const float *in, long long in_pair_stride, const QuadWork *work, int nquads,
+                        float *bc, float *br, long long vol, const FrameStrides &fr, int view, int x0,
+                        cudaStream_t st) {
+  const size_t smem = (size_t)4 * g.bp_s4 * sizeof(float4);
+  auto k = bp_kernel<ACC, MULTI>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  k<<<(unsigned)nwork * fr.n, NT, smem, st>>>(g, reinterpret_cast<const float4 *>(in), in_pair_stride / 4, work, bc,
-                                              br, vol, fr, 0, 0, rlog);
+  // launches that do not fill the chip share each quad among several CTAs
+  const long long quads = (long long)nquads * fr.n;
+  const int split = (int)std::max<long long>(1, std::min<long long>(4, (4 * 148 + quads - 1) / quads));
+  k<<<(unsigned)(quads * split), kBpThreads<ACC>, smem, st>>>(g, reinterpret_cast<const float4 *>(in), in_pair_stride / 4,
+                                                         work, bc, br, vol, fr, view, x0, split);
   return cudaGetLastError();
 }
 
 cudaError_t launch_bp(const DevGeom &g, const float *in, long long in_pair_stride, const QuadWork *work, int nwork,
-                      float *bc, float *br, long long vol, const ProjTune &tune, const FrameStrides &fr,
-                      cudaStream_t st) {
+                      float *bc, float *br, long long vol, const FrameStrides &fr, cudaStream_t st) {
   if (nwork <= 0 || fr.n <= 0) return cudaSuccess;
-  const int kb = tune.bp_planes > 0 ? tune.bp_planes : kBpZ;
-  // 384 threads (two CTAs of 80 registers per SM) measured faster than 256
-  // (three CTAs) at span 3 and 9 on B200: 1.58 vs 1.74 ms and 0.71 vs 0.74 ms
-  const int nt = tune.bp_threads > 0 ? tune.bp_threads : 384;
-  const int rl = bp_tile_log2(g, tune);
-  if (rl < 0) return cudaErrorInvalidValue;
-  if (kb == 8 && nt == 256) return launch_bp_t<8, 256>(g, in, in_pair_stride, work, nwork, bc, br, vol, fr, rl, st);
-  if (kb == 8 && nt == 384) return launch_bp_t<8, 384>(g, in, in_pair_stride, work, nwork, bc, br, vol, fr, rl, st);
-  if (kb == 4 && nt == 256) return launch_bp_t<4, 256>(g, in, in_pair_stride, work, nwork, bc, br, vol, fr, rl, st);
-  if (kb == 4 && nt == 384) return launch_bp_t<4, 384>(g, in, in_pair_stride, work, nwork, bc, br, vol, fr, rl, st);
-  return cudaErrorInvalidValue;
+  auto f = fr.n > 1 ? launch_bp_t<false, true> : launch_bp_t<false, false>;
+  return f(g, in, in_pair_stride, work, nwork, bc, br, vol, fr, 0, 0, st);
 }
 
 cudaError_t launch_adj(const DevGeom &g, const float *in, long long in_pair_stride, const QuadWork *work, int nwork,
                        float *bc, float *br, long long vol, const FrameStrides &fr, cudaStream_t st) {
   if (nwork <= 0 || fr.n <= 0) return cudaSuccess;
   const size_t smem = (size_t)g.bp_splanes * sizeof(float4);
-  auto k = adj_kernel<kBpZ>;
+  auto k = adj_kernel<kAdjZ>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -1541,15 +1599,7 @@ cudaError_t launch_adj_rotate(const DevGeom &g, const int *pair_views, int npair
 cudaError_t launch_bp_sum(const DevGeom &g, const float *quad, int view, int x0, int nquads, float *out,
                           cudaStream_t st) {
   if (nquads <= 0) return cudaSuccess;
-  const size_t smem = (size_t)g.bp_splanes * sizeof(float4);
-  auto k = bp_kernel<kBpZ, true>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (e != cudaSuccess) return e;
-  k<<<nquads, 256, smem, st>>>(g, reinterpret_cast<const float4 *>(quad), 0, nullptr, out, nullptr, 0, one_frame(), view,
-                               x0, bp_tile_log2(g, default_tune()));
-  return cudaGetLastError();
+  return launch_bp_t<true, false>(g, quad, 0, nullptr, nquads, out, nullptr, 0, one_frame(), view, x0, st);
 }
 
 cudaError_t launch_rotback(const DevGeom &g, const int *pair_views, int npairs, const float *bc, const float *br,

@@ -26,17 +26,15 @@ namespace hrrt {
 #ifndef HRRT_FP_SLOTS
 #define HRRT_FP_SLOTS 3
 #endif
-#ifndef HRRT_BP_MIN_BLOCKS
-#define HRRT_BP_MIN_BLOCKS 3
-#endif
 constexpr int kFpPlanes = 9;                   // default planes per forward-projection task (odd: bank-conflict free)
 constexpr int kFpSlots = HRRT_FP_SLOTS;       // sampled rows in flight between producers and consumers
 constexpr int kFpZPad = 16;     // zeroed entries after each sampled row
 constexpr int kFpEndPlanes = 4; // planes per end-plane task (they cost ~2x a middle plane)
 constexpr int kFpMaxGroups = 32; // segment groups the forward projector stages per row (22 at span 3)
-constexpr int kBpZ = 8;         // z per back-projection task
-constexpr int kBpMinBlocks = HRRT_BP_MIN_BLOCKS;  // resident back-projection CTAs per SM (register budget)
-constexpr int kBpPad = 8;       // zero planes on each side of a segment in the back projector (>= kBpZ)
+constexpr int kBpZ = 4;         // z per back-projection task
+constexpr int kBpRows = 4;      // rotated rows per back-projection task (rows kBpRows*m .. kBpRows*m+3)
+constexpr int kAdjZ = 8;        // z per task of the exact adjoint
+constexpr int kBpPad = 8;       // zero planes on each side of a segment in the back projector
 constexpr int kAdjCover = 8;    // rotated-frame points whose bilinear footprint covers a voxel (at most 5 on HRRT)
 
 struct FpTask {
@@ -58,6 +56,22 @@ struct BpLut {   // blookup (sbrt:672-700) in direct form: yr = z + d for z in [
   float f;
 };
 
+// One side of a segment group in the back projection of a row group: the rows
+// read the segment at yr = z + shift with a fraction f (BpLut), and the shifts
+// of adjacent rows differ by less than one plane, so that the four rows share
+// a window that starts at the smallest shift d.  With W[k] = p[z + d + k] and
+// D[k] = W[k+1] - W[k], a row whose shift is d + 1 takes W[1] + f*D[1], one
+// whose shift is d takes W[1] + (f-1)*D[0].  Along the rows the shift falls on
+// side 0 and rises on side 1, so the rows at d + 1 are the first or the last k.
+struct __align__(16) BpRows {
+  int16_t off[4];  // shared slot of plane d + k, from that of plane 0 (bp_slot)
+  int16_t zs, ze;  // planes any of the rows takes anything from
+  int32_t k;       // rows at d + 1 (0..3), or kBpWide: evaluated row by row
+  float u[4];      // f or f - 1
+};
+
+constexpr int kBpWide = 4;
+
 struct DevGeom {
   int nx, nz, zp, c, nseg, groupmax, zshift, segmentsize, pplanes, nviews, nquads;
   int fov_columns, z_min, z_max;
@@ -77,6 +91,7 @@ struct DevGeom {
   int *adj_cnt;                     //   rotated-frame points (index, weight bits) [.][kAdjCover], their count
   int adj_pairs;                    //   pair slots the two buffers hold (for every image column)
   const BpLut *bplut;               // [groupmax][ny]
+  const BpRows *bprows;             // [c / kBpRows + 1][groupmax][2 sides]: side 0 rows y, side 1 rows ny - y
   const int16_t *nzmask;            // [nviews/2][nquads]
   const float *sin_psi, *cos_psi;   // [nviews]
   const short2 *fov_xy;             // [fov_columns]
@@ -89,7 +104,7 @@ struct DevGeom {
   int *range_err;                   // non-zero after an input exceeded the fp16 range (HRRT_STORE_F16)
   const int *bp_soff;               // [nseg] back projector: shared-memory plane of yr_bottom
   const int *bp_src;                // [bp_splanes] quad-layout plane of each shared plane, -1 = zero
-  int bp_splanes;
+  int bp_splanes, bp_s4;            // their number; shared slots per phase (bp_slot)
 };
 
 struct QuadWork {  // one (view pair slot, quad) work item
@@ -124,11 +139,11 @@ inline FrameStrides one_frame() { return FrameStrides{1, nullptr, 0, 0, 0, 0, 0}
 struct ProjTune {
   int fp_planes;  // planes per forward-projection task: 7, 9 or 11 (0: kFpPlanes)
   int fp_pwarps;  // producer warps of the forward projector (0: as many as fit, 2..6)
-  int bp_planes;  // planes per back-projection task: 4 or 8 (0: kBpZ)
-  int bp_threads; // threads per back-projection CTA: 256 or 384 (0: 384)
-  int bp_tile;    // back projection: plane runs side by side in a warp's 32 tasks, a power of 2
-                  // up to 32 (the rest of the warp takes consecutive rows; 0: 2 above 12
-                  // segment groups, else 4)
+  // the back projector has one shape (a row group of kBpRows rows x kBpZ planes a
+  // thread); these are checked and kept, and choose nothing
+  int bp_planes;  // 4 or 8 (0: 8)
+  int bp_threads; // 256 or 384 (0: 384)
+  int bp_tile;    // a power of 2 up to 32
 };
 inline ProjTune default_tune() { return ProjTune{0, 0, 0, 0, 0}; }
 constexpr int kFpPlaneVariants[3] = {7, 9, 11};
@@ -144,8 +159,7 @@ cudaError_t launch_fp(const DevGeom &g, const float *image, const QuadWork *work
                       const ProjTune &tune, const FrameStrides &fr, cudaStream_t st);
 // back projection of quad-layout input into the column (Bc) / row (Br) partials
 cudaError_t launch_bp(const DevGeom &g, const float *in, long long in_pair_stride, const QuadWork *work, int nwork,
-                      float *bc, float *br, long long vol, const ProjTune &tune, const FrameStrides &fr,
-                      cudaStream_t st);
+                      float *bc, float *br, long long vol, const FrameStrides &fr, cudaStream_t st);
 // exact adjoint of the forward projector: z-transpose into the column / row
 // partials (rows scaled as the forward projector scales them)
 cudaError_t launch_adj(const DevGeom &g, const float *in, long long in_pair_stride, const QuadWork *work, int nwork,

@@ -269,11 +269,9 @@ int hrrt_reset_kernel_stats(hrrt_ctx *ctx);
 typedef struct hrrt_tuning {
   int fp_planes;          /* planes per forward-projection task: 7, 9 or 11 (0: 9) */
   int fp_producer_warps;  /* sampling warps of the forward projector: 2..6 (0: as many as fit) */
-  int bp_planes;          /* planes per back-projection task: 4 or 8 (0: 8) */
-  int bp_threads;         /* threads per back-projection CTA: 256 or 384 (0: 384) */
-  int bp_tile;            /* back projection: plane runs side by side in a warp, a power of 2 up to 32;
-                             the warp's other tasks take consecutive rows (0: 2 above 12 segment
-                             groups, else 4) */
+  int bp_planes;          /* 4 or 8 (0: 8), bp_threads 256 or 384 (0: 384), bp_tile a power of 2 up to 32 (0: */
+  int bp_threads;         /* the library's): checked and kept; the back projector has one shape */
+  int bp_tile;
   double fp_ms, bp_ms;    /* filled by the tuners: the chosen shapes' device time per launch */
 } hrrt_tuning;
 
