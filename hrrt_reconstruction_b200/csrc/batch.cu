@@ -33,7 +33,7 @@ struct hrrt_batch {
   float *images = nullptr;                      // [frame][vol]
   double *sums = nullptr;                       // [frame]
   int group = 1;                                // frames per launch
-  float *ratio = nullptr, *bc = nullptr, *br = nullptr;  // scratch of one group
+  float *ratio = nullptr, *bc = nullptr, *br = nullptr, *samples = nullptr;  // scratch of one group
   double *partial = nullptr;                    // [group][pb]
   int pb = 0;
   int *d_order = nullptr;                       // [nframes] frames by descending iteration count
@@ -64,10 +64,11 @@ struct hrrt_batch {
                         (long long)in_elems,
                         (long long)ctx->npairs * ctx->quad_pair,
                         (long long)ctx->npairs * ctx->vol,
-                        (long long)pb};
+                        (long long)pb,
+                        (long long)ctx->npairs * ctx->dg.samp_pair * 4};
   }
   SubsetBufs bufs(int start, int n) const {
-    return SubsetBufs{images, q_prompts, q_add, ratio, bc, br, strides(start, n)};
+    return SubsetBufs{images, q_prompts, q_add, ratio, bc, br, samples, strides(start, n)};
   }
 };
 
@@ -116,7 +117,7 @@ int autotune(hrrt_ctx *ctx, const SubsetBufs &bb, int repeats, hrrt_tuning *chos
   double best_fp = 1e30, best_bp = 1e30;
   for (int vi = 0; vi < 3; vi++) {
     if (!ctx->d_fptasks[vi]) continue;
-    const int cwarps = (ctx->nfptasks[vi] + 31) / 32;
+    const int cwarps = ctx->fp_offer_warps[vi];
     for (int pw : {2, 3, 4, 6}) {
       if (cwarps + pw > kFpVariantWarps[vi]) continue;
       ProjTune t = saved;
@@ -126,8 +127,8 @@ int autotune(hrrt_ctx *ctx, const SubsetBufs &bb, int repeats, hrrt_tuning *chos
       const DevGeom &g = adj ? ctx->dg_adj : ctx->dg;
       double ms = 0;
       int rc = time_launch(ctx, repeats, [&] {
-        return launch_fp(g, bb.image, fw, ctx->fp_cnt[s], 1, bb.prompts, bb.add, ctx->storage, bb.ratio,
-                         ctx->quad_pair, t, bb.fr, ctx->stream);
+        return launch_fp(g, bb.image, bb.samples, ctx->d_pair_views + (size_t)s * ctx->npairs, 0, ctx->npairs, fw, ctx->fp_cnt[s], 1, bb.prompts, bb.add, ctx->storage, bb.ratio,
+                         ctx->quad_pair, bb.fr, ctx->stream);
       }, &ms);
       if (rc) {
         apply_tune(ctx, saved);
@@ -321,7 +322,8 @@ int hrrt_batch_create(hrrt_ctx *ctx, int nframes, int storage, const float *norm
   if (!b->d_order) return bail(fail(ctx, HRRT_ERR_NOMEM, "batch: frame inputs"));
   // frames per launch: as many as the free memory holds (2 GiB kept back)
   b->pb = post_iteration_blocks(ctx->dg);
-  const size_t per = sizeof(float) * ((size_t)ctx->npairs * ctx->quad_pair + 2 * (size_t)ctx->npairs * ctx->vol) +
+  const size_t samp = (size_t)ctx->npairs * ctx->dg.samp_pair * 4;
+  const size_t per = sizeof(float) * ((size_t)ctx->npairs * ctx->quad_pair + 2 * (size_t)ctx->npairs * ctx->vol + samp) +
                      sizeof(double) * (size_t)b->pb;
   size_t free_b = 0, total_b = 0;
   CK(cudaMemGetInfo(&free_b, &total_b), "batch");
@@ -331,7 +333,8 @@ int hrrt_batch_create(hrrt_ctx *ctx, int nframes, int storage, const float *norm
   b->ratio = b->alloc<float>((size_t)b->group * ctx->npairs * ctx->quad_pair, &e);
   b->bc = b->ratio ? b->alloc<float>((size_t)b->group * ctx->npairs * ctx->vol, &e) : nullptr;
   b->br = b->bc ? b->alloc<float>((size_t)b->group * ctx->npairs * ctx->vol, &e) : nullptr;
-  b->partial = b->br ? b->alloc<double>((size_t)b->group * b->pb, &e) : nullptr;
+  b->samples = b->br ? b->alloc<float>((size_t)b->group * samp, &e) : nullptr;
+  b->partial = b->samples ? b->alloc<double>((size_t)b->group * b->pb, &e) : nullptr;
   if (!b->partial) return bail(fail(ctx, HRRT_ERR_NOMEM, "batch: scratch"));
   ctx->batch = b;
   ctx->have_inputs = false;  // the context's single-frame inputs are replaced

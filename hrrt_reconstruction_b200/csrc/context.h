@@ -37,6 +37,7 @@ struct hrrt_ctx {
   float *d_image = nullptr;
   float *d_nfinv = nullptr;
   float *d_ratio = nullptr, *d_bc = nullptr, *d_br = nullptr;
+  float *d_samples = nullptr;   // the forward projector's rotated rows, [npairs][samp_pair][4]
   float *d_tmp_img = nullptr;  // test entry points
   float *d_rows = nullptr;
   double *d_partial = nullptr, *d_sum = nullptr;
@@ -51,7 +52,8 @@ struct hrrt_ctx {
   // each plane variant (null where the variant does not fit the geometry)
   hrrt::ProjTune tune = hrrt::default_tune();
   hrrt::FpTask *d_fptasks[3] = {nullptr, nullptr, nullptr};
-  int nfptasks[3] = {0, 0, 0};
+  int nfptasks[3] = {0, 0, 0}, fp_run[3] = {0, 0, 0};
+  int fp_offer_warps[3] = {0, 0, 0};  // warps the variant's offer counts (kFpVariantWarps)
   bool have_inputs = false, have_sens = false, have_image = false;
 
   // chunked upload: flat-file planes staged through two device buffers, the
@@ -197,7 +199,7 @@ inline void drain_timers(hrrt_ctx *ctx) {
 struct SubsetBufs {
   float *image;
   const void *prompts, *add;
-  float *ratio, *bc, *br;
+  float *ratio, *bc, *br, *samples;
   FrameStrides fr;
 };
 

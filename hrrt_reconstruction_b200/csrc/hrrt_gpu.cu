@@ -59,66 +59,81 @@ std::vector<float> psf_taps(float fwhm1, float fwhm2, float ratio, float pixel_s
   return k;
 }
 
-// Forward-projection tasks shared by every quad: (segment, plane run, kind).
-std::vector<FpTask> build_fp_tasks(const Geometry &g, int PL) {
-  std::vector<FpTask> mid, ends;
-  for (int p0 = 0; p0 < g.nz; p0 += PL) mid.push_back(FpTask{0, (int16_t)p0, (int16_t)std::min(PL, g.nz - p0), 0});
+// Warps of one thread per (segment, run of `planes` planes, kind), each kind
+// in whole warps: the rule by which a plane variant is offered.
+int fp_offer_warps(const Geometry &g, int planes) {
+  auto warps = [](int threads) { return (threads + 31) / 32; };
+  auto runs = [&](int n) { return (n + planes - 1) / planes; };
+  int mid = 0, ends = 0;
   for (int s = 1; s < g.nseg; s++) {
-    const int ns = g.yr_top[s] - g.yr_bottom[s] + 1;
-    for (int p0 = g.zshift; p0 < ns - g.zshift; p0 += PL)
-      mid.push_back(FpTask{(int16_t)s, (int16_t)p0, (int16_t)std::min(PL, ns - g.zshift - p0), 1});
-    // an end-plane run stays inside one end region, so its lookup entries are consecutive
-    for (int p0 = 0; p0 < g.zshift; p0 += kFpEndPlanes)
-      ends.push_back(FpTask{(int16_t)s, (int16_t)p0, (int16_t)std::min(kFpEndPlanes, g.zshift - p0), 2});
-    for (int p0 = ns - g.zshift; p0 < ns; p0 += kFpEndPlanes)
-      ends.push_back(FpTask{(int16_t)s, (int16_t)p0, (int16_t)std::min(kFpEndPlanes, ns - p0), 2});
+    mid += runs(g.yr_top[s] - g.yr_bottom[s] + 1 - 2 * g.zshift);
+    ends += 2 * ((g.zshift + 3) / 4);
   }
-  // one task kind per warp (the kinds cost different amounts per row, and a
-  // warp mixing them would set the pace of every row barrier): pad each kind
-  // to a multiple of 32 with empty tasks
-  std::vector<FpTask> t0, t1;
-  for (const FpTask &t : mid) (t.type == 0 ? t0 : t1).push_back(t);
+  return warps(runs(g.nz)) + warps(mid) + warps(ends);
+}
+
+// Forward-projection tasks shared by every quad.  Two threads share a task, 16
+// tasks make a warp, and a warp's tasks are of one kind (the kinds cost
+// different amounts per row): each kind is padded to whole warps.  The middle
+// planes' shared loads are served 16 threads (8 tasks) at a time: 4 runs of a
+// segment and the same runs of its mirror segment, which read the same planes
+// of the other half of a row, fall in 8 different bank groups (runs of an odd
+// number of planes, rows 4 modulo 8 entries long).  What does not fill such
+// eights comes last.
+std::vector<FpTask> build_fp_tasks(const Geometry &g, int PL) {
+  std::vector<FpTask> t0, eights, rest, ends;
+  for (int p0 = 0; p0 < g.nz; p0 += PL) t0.push_back(FpTask{0, (int16_t)p0, (int16_t)std::min(PL, g.nz - p0), 0});
+  for (int s = 1; s < g.nseg; s += 2) {
+    const int mid_end = g.yr_top[s] - g.yr_bottom[s] + 1 - g.zshift;
+    const int runs = (mid_end - g.zshift + PL - 1) / PL;
+    for (int r0 = 0; r0 < runs; r0 += 4) {
+      auto &to = r0 + 3 <= runs ? eights : rest;  // three runs: an empty one fills the four
+      for (int sg = s; sg < s + 2; sg++)
+        for (int r = r0; r < (r0 + 3 <= runs ? r0 + 4 : runs); r++) {
+          const int p0 = g.zshift + r * PL;
+          to.push_back(r < runs ? FpTask{(int16_t)sg, (int16_t)p0, (int16_t)std::min(PL, mid_end - p0), 1}
+                                : FpTask{0, 0, 0, -1});
+        }
+    }
+    for (int sg = s; sg < s + 2; sg++)
+      for (int i0 = 0; i0 < 2 * g.zshift; i0 += kFpEndPlanes)
+        ends.push_back(FpTask{(int16_t)sg, (int16_t)i0, (int16_t)std::min(kFpEndPlanes, 2 * g.zshift - i0), 2});
+  }
+  eights.insert(eights.end(), rest.begin(), rest.end());
   std::vector<FpTask> out;
-  for (auto *lst : {&t0, &t1, &ends}) {
+  for (auto *lst : {&t0, &eights, &ends}) {
     out.insert(out.end(), lst->begin(), lst->end());
-    while (out.size() % 32) out.push_back(FpTask{0, 0, 0, -1});
+    while (out.size() % 16) out.push_back(FpTask{0, 0, 0, -1});
   }
   return out;
 }
 
 // Every shared-memory index the forward projector can form for this geometry
-// must lie inside the staged column; checked once here so the kernel needs no
-// run-time guards.
-std::string validate_fp(const Geometry &g, const std::vector<FpMid> &mid, const std::vector<FpTask> &tasks, int PL) {
-  const int ZS = g.zp + kFpZPad, FS = g.flookup_stride();
+// must lie inside the sampled row; checked once here so the kernel needs no
+// run-time guards.  `row`: its entries, of which kFpZPad are zeroes (16 where
+// only the planes of `PL`-plane runs are looked at, for the variant's offer).
+std::string validate_fp(const Geometry &g, const std::vector<FpMid> &mid, int PL, int row) {
+  const int FS = g.flookup_stride();
   int ymin = g.c;
   for (int x = 1; x <= g.c; x++)
     if (g.cyl0[x] != g.cyl1[x]) ymin = std::min<int>(ymin, g.cyl0[x]);
-  for (int y = ymin; y < g.c; y++) {
-    for (const FpTask &t : tasks) {
-      if (t.type < 0) continue;
-      if (t.type == 0) {
-        if (t.p0 + PL >= ZS) return "fp: segment-0 window out of range";
-        continue;
-      }
-      const int gg = (t.seg + 1) / 2 - 1;
+  for (int p0 = 0; p0 < g.nz; p0 += PL)
+    if (p0 + PL >= row) return "fp: segment-0 window out of range";
+  for (int y = ymin; y < g.c; y++)
+    for (int s = 1; s < g.nseg; s++) {
+      const int gg = (s + 1) / 2 - 1, ns = g.yr_top[s] - g.yr_bottom[s] + 1;
       const FpMid m = mid[(size_t)y * g.groupmax + gg];
       if (m.z < 0) continue;
-      if (t.type == 1) {
-        const int za = m.z + t.p0 - g.zshift, zb = m.z2 + t.p0 - g.zshift;
-        if (za < 0 || zb < 0 || za + PL >= ZS || zb + PL >= ZS) return "fp: middle window out of range";
-      } else {
-        const int ns = g.yr_top[t.seg] - g.yr_bottom[t.seg] + 1;
-        for (int j = 0; j < t.n; j++) {
-          const int r = t.p0 + j;
-          const int yri = (r < g.zshift) ? r : r - ns + 2 * g.zshift;
-          const int li = gg * 2 * g.zshift + yri;
-          const int z = g.fl_zzi[(size_t)y * FS + li], z2 = g.fl_zzi[(size_t)(g.ny - y) * FS + li];
-          if (z < 0 || z2 < 0 || z + 1 >= ZS || z2 + 1 >= ZS) return "fp: end-plane index out of range";
-        }
+      for (int p0 = g.zshift; p0 < ns - g.zshift; p0 += PL) {
+        const int za = m.z + p0 - g.zshift, zb = m.z2 + p0 - g.zshift;
+        if (za < 0 || zb < 0 || za + PL >= row || zb + PL >= row) return "fp: middle window out of range";
+      }
+      for (int i = 0; i < 2 * g.zshift; i++) {
+        const int li = gg * 2 * g.zshift + i;
+        const int z = g.fl_zzi[(size_t)y * FS + li], z2 = g.fl_zzi[(size_t)(g.ny - y) * FS + li];
+        if (z < 0 || z2 < 0 || z + 1 >= row || z2 + 1 >= row) return "fp: end-plane index out of range";
       }
     }
-  }
   return std::string();
 }
 
@@ -204,7 +219,7 @@ int build_work_lists(hrrt_ctx *ctx) {
 }
 
 SubsetBufs ctx_bufs(hrrt_ctx *ctx) {
-  return SubsetBufs{ctx->d_image, ctx->q_prompts, ctx->q_add, ctx->d_ratio, ctx->d_bc, ctx->d_br, one_frame()};
+  return SubsetBufs{ctx->d_image, ctx->q_prompts, ctx->q_add, ctx->d_ratio, ctx->d_bc, ctx->d_br, ctx->d_samples, one_frame()};
 }
 
 int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
@@ -227,8 +242,8 @@ int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
     }
     {
       Launch L(ctx, "fp_kernel");
-      CK(launch_fp(g, proj, fw, ctx->fp_cnt[s], 1, b.prompts, b.add, ctx->storage, b.ratio, ctx->quad_pair,
-                   ctx->tune, b.fr, ctx->stream),
+      CK(launch_fp(g, proj, b.samples, pv, 0, ctx->npairs, fw, ctx->fp_cnt[s], 1, b.prompts, b.add, ctx->storage, b.ratio, ctx->quad_pair,
+                   b.fr, ctx->stream),
          "fp_kernel");
     }
     if (adj) {
@@ -267,8 +282,8 @@ int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
     if (int rc = run_psf(ctx, b.image, ctx->d_image_psf)) return rc;
     {
       Launch L(ctx, "fp_kernel");
-      CK(launch_fp(g, ctx->d_image_psf, fw, ctx->fp_cnt[s], 1, b.prompts, b.add, ctx->storage, b.ratio,
-                   ctx->quad_pair, ctx->tune, b.fr, ctx->stream),
+      CK(launch_fp(g, ctx->d_image_psf, b.samples, pv, 0, ctx->npairs, fw, ctx->fp_cnt[s], 1, b.prompts, b.add, ctx->storage, b.ratio,
+                   ctx->quad_pair, b.fr, ctx->stream),
          "fp_kernel");
     }
     if (adj) {
@@ -292,8 +307,8 @@ int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
   }
   {
     Launch L(ctx, "fp_kernel");
-    CK(launch_fp(g, b.image, fw, ctx->fp_cnt[s], 1, b.prompts, b.add, ctx->storage, b.ratio, ctx->quad_pair,
-                 ctx->tune, b.fr, ctx->stream),
+    CK(launch_fp(g, b.image, b.samples, pv, 0, ctx->npairs, fw, ctx->fp_cnt[s], 1, b.prompts, b.add, ctx->storage, b.ratio, ctx->quad_pair,
+                 b.fr, ctx->stream),
        "fp_kernel");
   }
   if (adj) {
@@ -496,8 +511,8 @@ int apply_tune(hrrt_ctx *ctx, const ProjTune &t) {
   for (int i = 0; i < 3; i++)
     if (kFpPlaneVariants[i] == pl) vi = i;
   if (vi < 0 || !ctx->d_fptasks[vi]) return fail(ctx, HRRT_ERR_ARG, "tuning: plane variant unavailable for this geometry");
-  const int cwarps = (ctx->nfptasks[vi] + 31) / 32;
-  if (t.fp_pwarps != 0 && (t.fp_pwarps < 2 || t.fp_pwarps > 6 || cwarps + t.fp_pwarps > kFpVariantWarps[vi]))
+  if (t.fp_pwarps != 0 &&
+      (t.fp_pwarps < 2 || t.fp_pwarps > 6 || ctx->fp_offer_warps[vi] + t.fp_pwarps > kFpVariantWarps[vi]))
     return fail(ctx, HRRT_ERR_ARG, "tuning: producer warps out of range");
   if (t.bp_planes != 0 && t.bp_planes != 4 && t.bp_planes != 8)
     return fail(ctx, HRRT_ERR_ARG, "tuning: back-projection planes must be 4 or 8");
@@ -509,6 +524,7 @@ int apply_tune(hrrt_ctx *ctx, const ProjTune &t) {
   ctx->config_epoch++;
   ctx->dg.fptasks = ctx->dg_adj.fptasks = ctx->d_fptasks[vi];
   ctx->dg.nfptasks = ctx->dg_adj.nfptasks = ctx->nfptasks[vi];
+  ctx->dg.fp_run = ctx->dg_adj.fp_run = ctx->fp_run[vi];
   return HRRT_OK;
 }
 
@@ -688,15 +704,21 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
         const int z_lo = (zs / kBpZ) * kBpZ, z_hi = (ze / kBpZ) * kBpZ + kBpZ - 1;
         if (wide || z_lo + lo < yb - kBpPad || z_hi + lo + 2 > yt + kBpPad) e.k = kBpWide;
       }
-  // forward-projection task lists of every plane variant (one task per
-  // consumer thread, two producer warps at least); the default variant must
-  // fit, the others are offered to the tuner where they do
+  // forward-projection task lists of every plane variant; the default variant
+  // must be on offer, the others are for the tuner where they are
   std::vector<FpTask> vtasks[3];
   for (int i = 0; i < 3; i++) {
-    vtasks[i] = build_fp_tasks(g, kFpPlaneVariants[i]);
-    std::string vm = validate_fp(g, mid, vtasks[i], kFpPlaneVariants[i]);
-    if (vm.empty() && ((int)vtasks[i].size() + 31) / 32 + 2 > kFpVariantWarps[i])
-      vm = "fp: too many projection tasks for one CTA";
+    std::string vm = validate_fp(g, mid, kFpPlaneVariants[i], g.zp + 16);
+    ctx->fp_offer_warps[i] = fp_offer_warps(g, kFpPlaneVariants[i]);
+    if (vm.empty() && ctx->fp_offer_warps[i] + 2 > kFpVariantWarps[i]) vm = "fp: too many projection tasks for one CTA";
+    for (int k = i; k < 4 && vm.empty() && !ctx->fp_run[i]; k++) {
+      vtasks[i] = build_fp_tasks(g, kFpRuns[k]);
+      if (vtasks[i].size() / 16 + 1 <= kFpMaxWarps) {
+        vm = validate_fp(g, mid, kFpRuns[k], g.zp + kFpZPad);
+        ctx->fp_run[i] = kFpRuns[k];
+      }
+    }
+    if (vm.empty() && !ctx->fp_run[i]) vm = "fp: too many projection tasks for one CTA";
     if (!vm.empty()) {
       if (kFpPlaneVariants[i] == kFpPlanes) m = vm;
       vtasks[i].clear();
@@ -731,6 +753,7 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
   d.eps3 = g.sp.epsilon3;
   d.image_max = g.sp.image_max;
   d.unit = 1.0f;
+  d.unit2 = 0x3f8000003f800000ull;
   d.cyl0 = dupload(ctx, g.cyl0, &e);
   d.cyl1 = dupload(ctx, g.cyl1, &e);
   d.ybot = dupload(ctx, g.yr_bottom, &e);
@@ -780,6 +803,17 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
     d.adj_ent = dalloc<int2>(ctx, (size_t)ctx->npairs * g.nx * g.nx * kAdjCover, &e);
     d.adj_cnt = d.adj_ent ? dalloc<int>(ctx, (size_t)ctx->npairs * g.nx * g.nx, &e) : nullptr;
   }
+  // the forward projector's samples of a pair slot: per quad the centre column
+  // and two halves per rotated row
+  std::vector<int> samp_off(g.c + 1, 0);
+  d.samp_pair = d.samp_rows = 0;
+  for (int x = 1; x <= g.c; x++) {
+    if (g.cyl0[x] == g.cyl1[x]) continue;
+    samp_off[x] = d.samp_pair;
+    d.samp_pair += (1 + 2 * (g.c - g.cyl0[x])) * g.zp;
+    d.samp_rows = std::max(d.samp_rows, g.c - g.cyl0[x]);
+  }
+  d.samp_off = dupload(ctx, samp_off, &e);
   d.bplut = dupload(ctx, bpl, &e);
   d.bprows = dupload(ctx, bprows, &e);
   d.sin_psi = dupload(ctx, g.sin_psi, &e);
@@ -792,6 +826,7 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
     if (kFpPlaneVariants[i] == kFpPlanes) {
       d.fptasks = ctx->d_fptasks[i];
       d.nfptasks = ctx->nfptasks[i];
+      d.fp_run = ctx->fp_run[i];
     }
   }
   d.plane_seg = dupload(ctx, plane_seg, &e);
@@ -822,8 +857,9 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
   ctx->d_ratio = ctx->d_nfinv ? dalloc<float>(ctx, (size_t)ctx->npairs * ctx->quad_pair, &e) : nullptr;
   ctx->d_bc = ctx->d_ratio ? dalloc<float>(ctx, (size_t)ctx->npairs * ctx->vol, &e) : nullptr;
   ctx->d_br = ctx->d_bc ? dalloc<float>(ctx, (size_t)ctx->npairs * ctx->vol, &e) : nullptr;
+  if (ctx->d_br) ctx->d_samples = dalloc<float>(ctx, (size_t)ctx->npairs * d.samp_pair * 4, &e);
   const int pb = post_iteration_blocks(d);
-  ctx->d_partial = ctx->d_br ? dalloc<double>(ctx, pb, &e) : nullptr;
+  ctx->d_partial = ctx->d_samples ? dalloc<double>(ctx, pb, &e) : nullptr;
   ctx->d_sum = ctx->d_partial ? dalloc<double>(ctx, 1, &e) : nullptr;
   if (!ctx->d_sum) return bail(fail(ctx, HRRT_ERR_NOMEM, std::string("device allocation: ") + cudaGetErrorString(e)));
   // the adjoint runs with segment weights of 1 (its rows carry the forward
@@ -1226,7 +1262,7 @@ int hrrt_fp_pair(hrrt_ctx *ctx, const float *image_xyz, int view, float *prj) {
   CK(cudaMemcpyAsync(ctx->d_rows, prj, rows * 4, cudaMemcpyHostToDevice, ctx->stream), "fp_pair");
   {
     Launch L(ctx, "fp_kernel");
-    CK(launch_fp(ctx->dg, ctx->d_tmp_img, dw, (int)work.size(), 0, nullptr, nullptr, 0, ctx->d_ratio, ctx->quad_pair, ctx->tune, one_frame(), ctx->stream),
+    CK(launch_fp(ctx->dg, ctx->d_tmp_img, ctx->d_samples, nullptr, view, 1, dw, (int)work.size(), 0, nullptr, nullptr, 0, ctx->d_ratio, ctx->quad_pair, one_frame(), ctx->stream),
        "fp_kernel");
   }
   CK(launch_quad_to_rows(ctx->dg, g.nbins, ctx->d_ratio, dw, (int)work.size(), ctx->d_rows, ctx->stream), "unpack");
@@ -1275,7 +1311,8 @@ int hrrt_forward_project(hrrt_ctx *ctx, const float *image_xyz, float *sino) {
     const int cnt = off[b + 1] - off[b];
     {
       Launch L(ctx, "fp_kernel");
-      e = launch_fp(ctx->dg, ctx->d_tmp_img, dw + off[b], cnt, 0, nullptr, nullptr, 0, ctx->d_ratio, ctx->quad_pair, ctx->tune, one_frame(), ctx->stream);
+      e = launch_fp(ctx->dg, ctx->d_tmp_img, ctx->d_samples, nullptr, (int)b * ctx->npairs,
+                    std::min(ctx->npairs, V2 - (int)b * ctx->npairs), dw + off[b], cnt, 0, nullptr, nullptr, 0, ctx->d_ratio, ctx->quad_pair, one_frame(), ctx->stream);
     }
     if (e == cudaSuccess)
       e = launch_quad_to_file(ctx->dg, g.nbins, ctx->d_ratio, ctx->quad_pair, dw + off[b], cnt, dsino, ctx->stream);

@@ -6,8 +6,6 @@
 // bit-identical to the reference on the same inputs.
 #include "kernels.cuh"
 
-#include <cuda.h>  // CUtensorMap (the encoder is reached through the runtime's driver entry point)
-
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
@@ -24,16 +22,9 @@ __device__ __forceinline__ float4 operator+(float4 a, float4 b) {
 __device__ __forceinline__ float4 operator*(float4 a, float s) {
   return make_float4(a.x * s, a.y * s, a.z * s, a.w * s);
 }
-__device__ __forceinline__ float lane(const float4 &v, int l) {
-  return l == 0 ? v.x : (l == 1 ? v.y : (l == 2 ? v.z : v.w));
-}
 
 // ---- storage-type helpers for the sinogram inputs ----
 struct P4 { float v[4]; };
-__device__ __forceinline__ P4 load_p4(const int16_t *p, size_t i) {
-  const short4 s = reinterpret_cast<const short4 *>(p)[i];
-  return P4{{(float)s.x, (float)s.y, (float)s.z, (float)s.w}};
-}
 __device__ __forceinline__ P4 load_p4(const __half *p, size_t i) {
   const uint2 u = reinterpret_cast<const uint2 *>(p)[i];
   const __half2 a = *reinterpret_cast<const __half2 *>(&u.x);
@@ -49,6 +40,18 @@ __device__ __forceinline__ P4 load_p4(const __nv_bfloat16 *p, size_t i) {
   const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162 *>(&u.x);
   const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162 *>(&u.y);
   return P4{{__low2float(a), __high2float(a), __low2float(b), __high2float(b)}};
+}
+// lanes 0,1 or 2,3 of a quad: pair i of the array
+__device__ __forceinline__ float2 load_p2(const int16_t *p, size_t i) {
+  const short2 s = reinterpret_cast<const short2 *>(p)[i];
+  return make_float2((float)s.x, (float)s.y);
+}
+__device__ __forceinline__ float2 load_p2(const float *p, size_t i) { return reinterpret_cast<const float2 *>(p)[i]; }
+__device__ __forceinline__ float2 load_p2(const __half *p, size_t i) {
+  return __half22float2(reinterpret_cast<const __half2 *>(p)[i]);
+}
+__device__ __forceinline__ float2 load_p2(const __nv_bfloat16 *p, size_t i) {
+  return __bfloat1622float2(reinterpret_cast<const __nv_bfloat162 *>(p)[i]);
 }
 __device__ __forceinline__ void store_p4(int16_t *p, size_t i, const float *v) {
   reinterpret_cast<short4 *>(p)[i] = make_short4((short)v[0], (short)v[1], (short)v[2], (short)v[3]);
@@ -117,8 +120,6 @@ __device__ __forceinline__ Q2 ldq(const float4 *p) {
   return Q2{v.x, v.y};
 }
 __device__ __forceinline__ Q2 qadd(Q2 a, Q2 b) { return Q2{add2(a.lo, b.lo), add2(a.hi, b.hi)}; }
-__device__ __forceinline__ Q2 qmul(Q2 a, uint64_t s) { return Q2{mul2(a.lo, s), mul2(a.hi, s)}; }
-__device__ __forceinline__ Q2 qaddp(Q2 a, Q2 p, uint64_t one) { return Q2{addp(a.lo, p.lo, one), addp(a.hi, p.hi, one)}; }
 // packed a * b + c (one rounding), where no reference rounding order is to
 // be kept: the back projector (held to the reference within 2e-6, its sums
 // being incremental there and direct here) and the exact adjoint (held to
@@ -129,12 +130,8 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   return r;
 }
 __device__ __forceinline__ Q2 qfma(Q2 a, uint64_t b, Q2 c) { return Q2{fma2(a.lo, b, c.lo), fma2(a.hi, b, c.hi)}; }
-__device__ __forceinline__ float4 q2f(Q2 q) {
-  const float2 a = upk(q.lo), b = upk(q.hi);
-  return make_float4(a.x, a.y, b.x, b.y);
-}
 
-// ---- TMA bulk copies + mbarrier (sm_90+ async proxy) ----
+// ---- bulk copies + mbarriers (sm_90+ async proxy) ----
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -147,6 +144,9 @@ __device__ __forceinline__ void fence_mbar_init() {
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_tx(uint64_t *bar, uint32_t bytes) {
   asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
                "r"(bytes)
@@ -158,15 +158,12 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
-// one box of a 4-D tensor (coordinates innermost first) into shared memory,
-// completing on the mbarrier; the map is a __grid_constant__ kernel parameter
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
-                                            uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-      "%5}], [%6];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
-      : "memory");
+// whole 16-byte words of [p, p + bytes) brought into L2
+__device__ __forceinline__ void prefetch_l2(const void *p, size_t bytes) {
+  const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15;
+  const uintptr_t e = (reinterpret_cast<uintptr_t>(p) + bytes) & ~(uintptr_t)15;
+  if (e > a)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)(e - a)) : "memory");
 }
 // bounded wait on an mbarrier phase; on timeout records the error and returns false
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *err) {
@@ -217,351 +214,330 @@ __device__ __forceinline__ SamplePt sample_point(int a, int b, int c, int N, int
   s.base = (ix * N + iy) * zp;
   return s;
 }
-__device__ __forceinline__ float bilinear(const float *__restrict__ img, const SamplePt &s, int N, int zp, int z) {
-  if (s.base < 0) return 0.f;
-  const float r1 = __ldg(img + s.base + z);
-  const float r2 = __ldg(img + s.base + N * zp + z);
-  const float r3 = __ldg(img + s.base + zp + z);
-  const float r4 = __ldg(img + s.base + N * zp + zp + z);
-  return (r1 * s.c0 + r2 * s.c1) + (r3 * s.c2 + r4 * s.c3);
-}
-
 // ============================================================================
-// Forward projection (+ fused OP ratio), one CTA per (view pair, quad x).
-// Restates forward_proj3d_view1_thread (sbrt:1728-1978) for one x: the eight
-// symmetric rotated-grid columns at row y are sampled once into shared memory
-// (pam: lanes (x,y),(N-x,y),(N-y,x),(N-y,N-x); pam2: (x,N-y),(N-x,N-y),(y,x),
-// (y,N-x)), then every thread accumulates its own (segment, plane-run) outputs
-// for all four lanes, row by row in the reference's order.
-// The consumers are bound by instruction issue and shared-load latency (64
-// registers a thread at 1024 threads), not by shared-memory bandwidth.
-// Measured on B200 at span 3 and not used: rows staged as bf16 (half the
-// shared bytes, plus the widening: 1.89 -> 1.89 ms), consumer warps split
-// into two or three groups with a row-ready barrier each (2.12, 2.23 ms), and
-// two CTAs per quad with half the tasks each, two CTAs or one of 128
-// registers per SM (2.01, 3.27 ms).
+// Forward projection (+ fused OP ratio), restating forward_proj3d_view1_thread
+// (sbrt:1728-1978) for one (view pair, quad x) in two kernels:
+//   fp_sample_kernel : the eight symmetric rotated-grid columns at every row y
+//                      (pam: lanes (x,y),(N-x,y),(N-y,x),(N-y,N-x); pam2:
+//                      (x,N-y),(N-x,N-y),(y,x),(y,N-x)), the quad's lanes
+//                      interleaved; and the centre column (pam of y = c);
+//   fp_kernel        : every thread accumulates its own (segment, plane-run)
+//                      outputs, row by row in the reference's order.
+// Samples of a quad, entries of 4 lanes: [zp] centre column, then per row
+// y = cyl0[x] .. c-1 [2 halves][zp], at g.samp_off[x] of its pair slot.
+// fp_kernel is bound by shared memory (L1 87 % busy at span 3: 2 x 8 bytes for
+// 6 packed operations), fp_sample_kernel by the latency of its L2 reads.
+// Measured on B200, us a subset: span 3 1892 -> 1037 + 241, span 9 860 -> 475
+// + 241, a 24-ring scanner 53 -> 26 + 6; before, one kernel sampled with four
+// warps (bulk tensor copies of the corner columns) beside 28 warps of 9-plane
+// 4-lane tasks, whose accumulators and end-plane entries spilled.
+// Measured at span 3 and not used: sampling warps in fp_kernel with plain
+// loads (2151: too few in flight), all warps sampling 8 rows at a time (2497:
+// spills), runs of 17 planes without the order of build_fp_tasks (bank
+// conflicts 53 M -> 36 M, 1092 -> 1053).
 // ============================================================================
-// named barriers (id 0 is __syncthreads); ids are immediates so the kernel
-// reserves only the barriers it uses
-template <int ID>
-__device__ __forceinline__ void bar_sync_id(int count) {
-  asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(count) : "memory");
-}
-template <int ID>
-__device__ __forceinline__ void bar_arrive_id(int count) {
-  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "r"(count) : "memory");
-}
-// named barriers with immediate ids (a register id reserves all 16)
-__device__ __forceinline__ void bar_sync(int id, int count) {
-  switch (id) {
-    case 1: bar_sync_id<1>(count); break;
-    case 2: bar_sync_id<2>(count); break;
-    case 3: bar_sync_id<3>(count); break;
-    case 4: bar_sync_id<4>(count); break;
-    case 5: bar_sync_id<5>(count); break;
-    case 6: bar_sync_id<6>(count); break;
-    case 7: bar_sync_id<7>(count); break;
-    case 8: bar_sync_id<8>(count); break;
-    case 9: bar_sync_id<9>(count); break;
-    case 10: bar_sync_id<10>(count); break;
-    case 11: bar_sync_id<11>(count); break;
-    case 12: bar_sync_id<12>(count); break;
-    default: bar_sync_id<13>(count); break;
+// A warp takes one quad and half and `steps` rows, every other one; a CTA's
+// four warps are 2 quads x 2 rows at a time, whose points lie close together
+// in each of the four image regions they map to and share corner columns in
+// L1.  16 loads of 16 bytes in flight per lane (112 registers) and 16 rows a
+// warp measured 241 us for 9 span-3 pairs; 8-byte loads with twice the warps
+// 266, 4-byte loads 306, 4 x 4 tiles 270.
+constexpr int kSampleTile = 2;
+__global__ void __launch_bounds__(kSampleTile * kSampleTile * 32, 4)
+    fp_sample_kernel(DevGeom g, const float *__restrict__ image, const int *__restrict__ pair_views, int view0,
+                     int npairs, float4 *__restrict__ samples, FrameStrides fr, int steps) {
+  const int h = blockIdx.z & 1, frame = (blockIdx.z >> 1) / npairs, slot = (blockIdx.z >> 1) - frame * npairs;
+  const int wid = threadIdx.x >> 5, ln = threadIdx.x & 31, N = g.nx, c = g.c, zp = g.zp;
+  const int x = blockIdx.x * kSampleTile + 1 + wid % kSampleTile;
+  if (x > c) return;
+  const int ystart = g.cyl0[x];
+  if (ystart == g.cyl1[x]) return;
+  const int view = pair_views ? __ldg(pair_views + slot) : view0 + slot;
+  const float cosv = g.cos_psi[view], sinv = g.sin_psi[view];
+  const uint64_t one = g.unit2;
+  image += (size_t)(fr.map ? __ldg(fr.map + frame) : frame) * fr.image;
+  float4 *quad = samples + (size_t)frame * (fr.samples / 4) + (size_t)slot * g.samp_pair + g.samp_off[x];
+  const char *k1 = reinterpret_cast<const char *>(image), *k2 = k1 + (size_t)N * zp * 4;
+  const char *k3 = k1 + (size_t)zp * 4, *k4 = k2 + (size_t)zp * 4;
+  auto ld = [](const char *k, uint32_t o) { return __ldg(reinterpret_cast<const ulonglong2 *>(k + o)); };
+  const int y1 = blockIdx.y * kSampleTile * steps + wid / kSampleTile;
+  for (int y = y1; y < y1 + kSampleTile * steps; y += kSampleTile) {
+    // row y = c is the centre column: pam only
+    if (y < ystart || y > c || (y == c && h)) continue;
+    float4 *dst = quad + (y == c ? 0 : (size_t)(2 * (y - ystart) + 1 + h) * zp);
+    SamplePt pt;
+    {
+      const int l = ln & 3, yy = h ? N - y : y;
+      const int a = l == 0 ? x : l == 1 ? N - x : N - yy, b = l < 2 ? yy : l == 2 ? x : N - x;
+      pt = sample_point(a, b, c, N, zp, cosv, sinv);
+    }
+    // Four planes a lane: the corner columns (ix,iy), (ix+1,iy), (ix,iy+1),
+    // (ix+1,iy+1) of the four points in 16-byte loads, all in flight together,
+    // and the quad's 4 x 4 values in two 32-byte stores.
+    uint32_t o[4];
+    uint64_t wt[4][4];
+    bool in[4];
+#pragma unroll
+    for (int l = 0; l < 4; l++) {
+      const int b = __shfl_sync(0xffffffffu, pt.base, l);
+      in[l] = b >= 0;
+      o[l] = 4u * (uint32_t)max(b, 0);
+      auto dup = [&](float w) {
+        const float u = __shfl_sync(0xffffffffu, w, l);
+        return pk(u, u);
+      };
+      wt[l][0] = dup(pt.c0);
+      wt[l][1] = dup(pt.c1);
+      wt[l][2] = dup(pt.c2);
+      wt[l][3] = dup(pt.c3);
+    }
+    for (int z = 4 * ln; z < zp; z += 128) {
+      ulonglong2 c[4][4];
+#pragma unroll
+      for (int l = 0; l < 4; l++) {
+        c[l][0] = ld(k1, o[l] + 4u * z);
+        c[l][1] = ld(k2, o[l] + 4u * z);
+        c[l][2] = ld(k3, o[l] + 4u * z);
+        c[l][3] = ld(k4, o[l] + 4u * z);
+      }
+      float2 v[4][2];
+#pragma unroll
+      for (int l = 0; l < 4; l++) {
+        // sums in the reference's corner order; outside points sample as zero
+        const uint64_t a = add2(addp(mul2(c[l][0].x, wt[l][0]), mul2(c[l][1].x, wt[l][1]), one),
+                                addp(mul2(c[l][2].x, wt[l][2]), mul2(c[l][3].x, wt[l][3]), one));
+        const uint64_t b = add2(addp(mul2(c[l][0].y, wt[l][0]), mul2(c[l][1].y, wt[l][1]), one),
+                                addp(mul2(c[l][2].y, wt[l][2]), mul2(c[l][3].y, wt[l][3]), one));
+        v[l][0] = upk(in[l] ? a : 0ull);
+        v[l][1] = upk(in[l] ? b : 0ull);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+        asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + z + 2 * i), "f"(v[0][i].x),
+                     "f"(v[1][i].x), "f"(v[2][i].x), "f"(v[3][i].x), "f"(v[0][i].y), "f"(v[1][i].y), "f"(v[2][i].y),
+                     "f"(v[3][i].y)
+                     : "memory");
+    }
   }
 }
-__device__ __forceinline__ void bar_arrive(int id, int count) {
-  switch (id) {
-    case 1: bar_arrive_id<1>(count); break;
-    case 2: bar_arrive_id<2>(count); break;
-    case 3: bar_arrive_id<3>(count); break;
-    case 4: bar_arrive_id<4>(count); break;
-    case 5: bar_arrive_id<5>(count); break;
-    case 6: bar_arrive_id<6>(count); break;
-    case 7: bar_arrive_id<7>(count); break;
-    case 8: bar_arrive_id<8>(count); break;
-    case 9: bar_arrive_id<9>(count); break;
-    case 10: bar_arrive_id<10>(count); break;
-    case 11: bar_arrive_id<11>(count); break;
-    default: bar_arrive_id<12>(count); break;
-  }
-}
-constexpr int kBarFull = 1;                 // + slot: sampled row ready (producers arrive, consumers wait)
-constexpr int kBarEmpty = 1 + kFpSlots;     // + slot: sampled row consumed (consumers arrive, producers wait)
-constexpr int kBarProd = 1 + 2 * kFpSlots;  // producers only: corner slot read by every producer
-static_assert(kBarProd <= 13, "named barrier ids");
 
-template <int MODE, int PL, int MW, typename PT, typename AT>
-__global__ void __launch_bounds__(MW * 32, 1) fp_kernel(DevGeom g, const float *__restrict__ image,
+// a pair of lanes at a byte offset of the dynamic shared memory
+__device__ __forceinline__ uint64_t lds2(const float4 *P, int at) {
+  return *reinterpret_cast<const uint64_t *>(reinterpret_cast<const char *>(P) + at);
+}
+
+// One CTA per (view pair, quad x): one warp brings the rows in by bulk copies,
+// a ring of kFpSlots ahead; the others pass through them each at its own pace.
+template <int MODE, int PL, typename PT, typename AT>
+__global__ void __launch_bounds__(kFpMaxWarps * 32, 1) fp_kernel(DevGeom g, const float4 *__restrict__ samples,
                                                      const QuadWork *__restrict__ work,
                                                      const PT *__restrict__ prompts, const AT *__restrict__ add,
                                                      float4 *__restrict__ out, long long out_pair_stride,
-                                                     int nprod_warps, FrameStrides fr,
-                                                     const __grid_constant__ CUtensorMap cols, int use_cols) {
-  // shared memory: [S slots][8 points][2 column pairs][2*zp] staged corner
-  // columns, 2*cpair zeros (the corners of outside points), [S slots][2 halves]
-  // [ZS] sampled rows, [ZS] centre column (S = kFpSlots)
-  const uint64_t one = pk(g.unit, g.unit);
+                                                     FrameStrides fr) {
+  // shared memory: [kFpSlots][2 halves][ZS] sampled rows, [ZS] centre column,
+  // [kFpSlots][groupmax] the rows' middle-plane sampling entries
   extern __shared__ __align__(128) float4 smem[];
-  const int ZS = g.zp + kFpZPad;
-  const int zp = g.zp;
-  const int cpair = 2 * zp;  // floats per column pair
-  float *corners = reinterpret_cast<float *>(smem);
-  // the four corner columns of a point arrive as one box of the image's
-  // tensor map where the map is there and the slots are 128-byte aligned
-  const bool box4 = use_cols && (smem_u32(corners) & 127u) == 0;
-  const int zoff = kFpSlots * 8 * 2 * cpair;
-  float *zcol = corners + zoff;
-  float4 *rows = smem + (size_t)(kFpSlots * 8 * 2 + 2) * cpair / 4;  // [S][2][ZS]
-  float4 *cen = rows + 2 * kFpSlots * ZS;
-  __shared__ ulonglong2 s_w[kFpSlots][4][2];
-  __shared__ int s_off[kFpSlots][8];
-  // each row's middle-plane sampling entries (z, f, z2, f2 per group),
-  // copied in with the row's columns.  Twice as many slots as rows in flight:
-  // the entries of row r + S arrive while the consumers may still read those
-  // of rows r - S + 1 .. r.  (3 KB: two CTAs per SM still fit at span 9.)
-  __shared__ __align__(16) FpMid s_mid[2 * kFpSlots][kFpMaxGroups];
-  __shared__ __align__(8) uint64_t s_bar[kFpSlots];
+  const int ZS = g.zp + kFpZPad, zp = g.zp, G = g.groupmax;
+  const int row_bytes = 2 * ZS * 16;
+  float4 *cen = smem + 2 * kFpSlots * ZS;
+  FpMid *s_mid = reinterpret_cast<FpMid *>(cen + ZS);
+  __shared__ __align__(8) uint64_t s_full[kFpSlots], s_empty[kFpSlots], s_cen;
 
   const int nwork = gridDim.x / fr.n, frame = blockIdx.x / nwork, item = blockIdx.x - frame * nwork;
   const QuadWork w = work[item];
-  const int fs = fr.map ? __ldg(fr.map + frame) : frame;
-  image += (size_t)fs * fr.image;
-  out += (size_t)frame * fr.ratio / 4;
-  if (MODE == 1) {
-    prompts += (size_t)fs * fr.input;
-    add += (size_t)fs * fr.input;
-  }
-  const int x = w.x, v = w.view;
-  const int N = g.nx, c = g.c;
-  const float cosv = g.cos_psi[v], sinv = g.sin_psi[v];
-  const int ystart = g.cyl0[x];
-  const int nrows = c - ystart;
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int nprod = nprod_warps * 32;   // producer threads: [ncons, nthr)
-  const int ncons = nthr - nprod;        // consumer threads: one task each
-  const bool producer = tid >= ncons;
-  const int ptid = tid - ncons;
+  const int x = w.x, N = g.nx, ystart = g.cyl0[x], nrows = g.c - ystart;
+  const int tid = threadIdx.x, ln = tid & 31, ncons = (blockDim.x >> 5) - 1;
 
-  // TMA issue (producer lanes 0-7, one sample point each): the two contiguous
-  // column pairs (ix, iy..iy+1) and (ix+1, iy..iy+1) of each inside point
-  auto issue_row = [&](int r) {
-    const int sl = r % kFpSlots, y = ystart + r, l = ptid;
-    int a, b;
-    switch (l) {
-      case 0: a = x; b = y; break;
-      case 1: a = N - x; b = y; break;
-      case 2: a = N - y; b = x; break;
-      case 3: a = N - y; b = N - x; break;
-      case 4: a = x; b = N - y; break;
-      case 5: a = N - x; b = N - y; break;
-      case 6: a = y; b = x; break;
-      default: a = y; b = N - x; break;
-    }
-    const SamplePt pt = sample_point(a, b, c, N, zp, cosv, sinv);
-    const bool inside = pt.base >= 0;
-    // weights packed per lane pair: s_w[slot][point/2] = {(c0,c0'),(c1,c1')},{(c2,c2'),(c3,c3')}
-    float *wf = reinterpret_cast<float *>(&s_w[sl][l >> 1][0]);
-    const int e = l & 1;
-    wf[0 + e] = pt.c0;
-    wf[2 + e] = pt.c1;
-    wf[4 + e] = pt.c2;
-    wf[6 + e] = pt.c3;
-    // outside points read the zero column pairs
-    s_off[sl][l] = inside ? (sl * 8 + l) * 2 * cpair : zoff;
-    const unsigned m = __ballot_sync(0xffu, inside);
-    const int G = g.groupmax, es = r % (2 * kFpSlots);
-    if (l == 0) {
-      fence_proxy_async();
-      mbar_arrive_tx(&s_bar[sl], (uint32_t)__popc(m) * 2u * cpair * 4u + (uint32_t)G * 16u);
-    }
-    __syncwarp(0xffu);
-    if (l == 0) bulk_g2s(&s_mid[es][0], g.fpmid + (size_t)y * G, (uint32_t)G * 16u, &s_bar[sl]);
-    if (inside) {
-      float *dst = corners + ((size_t)(sl * 8 + l) * 2) * cpair;
-      const int ix = pt.base / (N * zp), iy = pt.base / zp - ix * N;
-      if (box4 && iy + 1 < N) {
-        // columns (ix, iy..iy+1) and (ix+1, iy..iy+1): box {zp, 2, 2} at
-        // (0, iy, ix, stored frame), laid out as the two pairs below
-        tma_load_4d(dst, &cols, 0, iy, ix, fs, &s_bar[sl]);
-      } else {
-        // the pair (ix, N-1..N) runs on into column (ix+1, 0) in the
-        // contiguous image, as the reference's flat addressing reads it
-        bulk_g2s(dst, image + pt.base, cpair * 4u, &s_bar[sl]);
-        bulk_g2s(dst + cpair, image + pt.base + (size_t)N * zp, cpair * 4u, &s_bar[sl]);
-      }
-    }
-  };
-
-  if (tid == 0) {
-#pragma unroll
-    for (int s = 0; s < kFpSlots; s++) mbar_init(&s_bar[s], 1);
+  if (tid < kFpSlots) {
+    mbar_init(&s_full[tid], 1);
+    mbar_init(&s_empty[tid], ncons);
+    if (tid == 0) mbar_init(&s_cen, 1);
     fence_mbar_init();
   }
-  for (int i = tid; i < (2 * kFpSlots + 1) * kFpZPad; i += nthr) {
-    const int col = i / kFpZPad, k = i % kFpZPad;
-    rows[col * ZS + zp + k] = f4(0.f);
-  }
-  for (int i = tid; i < 2 * cpair; i += nthr) zcol[i] = 0.f;
-  __syncthreads();
-  if (producer && ptid < 8) {
-    for (int r = 0; r < kFpSlots && r < nrows; r++) issue_row(r);
-  }
-
-  // centre column y = c (sbrt:1815-1853): lanes (x,c),(N-x,c),(c,x),(c,N-x)
-  {
-    SamplePt cp[4];
-#pragma unroll
-    for (int l = 0; l < 4; l++) {
-      const int a = (l == 0) ? x : (l == 1) ? N - x : c;
-      const int b = (l == 0 || l == 1) ? c : (l == 2) ? x : N - x;
-      cp[l] = sample_point(a, b, c, N, zp, cosv, sinv);
-    }
-    for (int z = tid; z < zp; z += nthr)
-      cen[z] = make_float4(bilinear(image, cp[0], N, zp, z), bilinear(image, cp[1], N, zp, z),
-                           bilinear(image, cp[2], N, zp, z), bilinear(image, cp[3], N, zp, z));
-  }
-  for (int z = zp + tid; z < ZS; z += nthr) cen[z] = f4(0.f);
+  // zeroes past the end of every sampled row and of the centre column
+  for (int i = tid; i < (2 * kFpSlots + 1) * kFpZPad; i += blockDim.x)
+    smem[(i / kFpZPad) * ZS + zp + i % kFpZPad] = f4(0.f);
   __syncthreads();
 
-  bool timed_out = false;
-  if (producer) {
-    // ---------------- producers: bilinear samples, kFpSlots rows ahead ----------------
-    const int hsplit = nprod / 2;
-    const int h_mine = ptid >= hsplit, z_mine = ptid - h_mine * hsplit;
-    for (int r = 0; r < nrows; r++) {
-      const int sl = r % kFpSlots;
-      if (!mbar_wait(&s_bar[sl], (uint32_t)((r / kFpSlots) & 1), g.err)) timed_out = true;
-      if (r >= kFpSlots) bar_sync(kBarEmpty + sl, nthr);  // consumers are done with row r-S
-      {
-        // lanes (0,1) and (2,3) of this half share nothing but the plane: each
-        // lane pair is evaluated with packed pairs, its weights pre-packed
-        float4 *rw = rows + (size_t)sl * 2 * ZS + h_mine * ZS;
-        for (int z = z_mine; z < zp; z += hsplit) {
-          uint64_t vv[2];
-#pragma unroll
-          for (int pp = 0; pp < 2; pp++) {
-            const int pt = h_mine * 4 + 2 * pp;
-            const ulonglong2 wa = s_w[sl][pt >> 1][0], wb = s_w[sl][pt >> 1][1];
-            const float *qa = corners + s_off[sl][pt], *qb = corners + s_off[sl][pt + 1];
-            // corner order of the reference: r1 (ix,iy), r2 (ix+1,iy), r3 (ix,iy+1), r4 (ix+1,iy+1)
-            const uint64_t r1 = pk(qa[z], qb[z]), r2 = pk(qa[cpair + z], qb[cpair + z]);
-            const uint64_t r3 = pk(qa[zp + z], qb[zp + z]), r4 = pk(qa[cpair + zp + z], qb[cpair + zp + z]);
-            vv[pp] = add2(addp(mul2(r1, wa.x), mul2(r2, wa.y), one), addp(mul2(r3, wb.x), mul2(r4, wb.y), one));
-          }
-          *reinterpret_cast<ulonglong2 *>(rw + z) = make_ulonglong2(vv[0], vv[1]);
-        }
-      }
-      bar_arrive(kBarFull + sl, nthr);
-      // every producer has finished reading corner slot sl: refill it with row r+S
-      bar_sync(kBarProd, nprod);
-      if (ptid < 8 && r + kFpSlots < nrows) issue_row(r + kFpSlots);
+  if (tid >= 32 * ncons) {
+    if (ln != 0) return;
+    const float4 *src = samples + (size_t)frame * (fr.samples / 4) + (size_t)w.slot * g.samp_pair + g.samp_off[x];
+    const uint32_t half = (uint32_t)zp * 16u, mids = (uint32_t)G * 16u;
+    mbar_arrive_tx(&s_cen, half);
+    bulk_g2s(cen, src, half, &s_cen);
+    src += zp;
+    if (MODE == 1) {
+      // the quad's prompts and additive terms, for the ratio at the end, into L2
+      const int fs = fr.map ? __ldg(fr.map + frame) : frame;
+      const size_t i0 = (size_t)fs * fr.input + 4 * ((size_t)w.view * g.nquads + x) * g.pplanes;
+      prefetch_l2(prompts + i0, 4 * (size_t)g.pplanes * sizeof(PT));
+      prefetch_l2(add + i0, 4 * (size_t)g.pplanes * sizeof(AT));
     }
-    if (timed_out) {
-      // results are void (the host reports the status word); give copies
-      // still in flight a bounded chance to land before the CTA exits
-      for (int r = max(0, nrows - kFpSlots); r < nrows; r++)
-        mbar_wait(&s_bar[r % kFpSlots], (uint32_t)((r / kFpSlots) & 1), nullptr);
+    for (int r = 0; r < nrows; r++, src += 2 * zp) {
+      const int sl = r & (kFpSlots - 1);
+      if (r >= kFpSlots && !mbar_wait(&s_empty[sl], (uint32_t)((r / kFpSlots - 1) & 1), g.err)) break;
+      fence_proxy_async();
+      mbar_arrive_tx(&s_full[sl], 2u * half + mids);
+      float4 *row = smem + (size_t)sl * 2 * ZS;
+      bulk_g2s(row, src, half, &s_full[sl]);
+      bulk_g2s(row + ZS, src + zp, half, &s_full[sl]);
+      bulk_g2s(s_mid + sl * G, g.fpmid + (size_t)(ystart + r) * G, mids, &s_full[sl]);
     }
+    // stay until the last copies have landed, whatever the consumers did
+    mbar_wait(&s_cen, 0, nullptr);
+    for (int r = max(0, nrows - kFpSlots); r < nrows; r++)
+      mbar_wait(&s_full[r & (kFpSlots - 1)], (uint32_t)((r / kFpSlots) & 1), nullptr);
     return;
   }
 
-  // ---------------- consumers: one task (segment, plane run) each ----------------
-  // accumulators start at the centre sample of their plane (the reference
-  // assigns the centre column before accumulating rows y < c)
-  Q2 acc[PL];
-  const FpTask tk = (tid < g.nfptasks) ? g.fptasks[tid] : FpTask{0, 0, 0, -1};
-  {
-    const int zb = (tk.type < 0) ? 0 : g.ybot[tk.seg] + tk.p0;
+  // Two threads a task, for lanes 2q and 2q + 1 of the quad; accumulators
+  // start at the centre sample of their plane (the reference assigns the
+  // centre column before accumulating rows y < c).
+  const uint64_t one = g.unit2;
+  const FpTask tk = g.fptasks[tid >> 1];
+  const int q8 = 8 * (tid & 1);
+  const int sg = tk.seg, gg = (sg + 1) / 2 - 1;
+  // a warp's tasks are of one kind but for empty ones at its end
+  const int kind = __shfl_sync(0xffffffffu, (int)tk.type, 0);
+  const int ybot = tk.type > 0 ? g.ybot[sg] : 0, ns = tk.type > 0 ? g.ytop[sg] - ybot + 1 : g.nz;
+  // segment 2k takes pam at z and pam2 at z2, segment 2k-1 the converse
+  const int oA = q8 + ((sg & 1) ? 16 * ZS : 0), oB = q8 + ((sg & 1) ? 0 : 16 * ZS);
+  const FpMid *mid = s_mid + (gg < 0 ? 0 : gg);
+  auto centre = [&](int p) { return lds2(cen, 16 * min(ybot + p, ZS - 1) + q8); };
+  auto next_row = [&](int r) { return mbar_wait(&s_full[r & (kFpSlots - 1)], (uint32_t)((r / kFpSlots) & 1), g.err); };
+  auto row_done = [&](int r) {
+    __syncwarp();
+    if (ln == 0) mbar_arrive(&s_empty[r & (kFpSlots - 1)]);
+  };
+  // n planes (plane_of(j), values val(j)) of the task's segment: scale
+  // (sbrt:1953-1975), then either store the estimate or the OP ratio
+  // (pt_update_est_w3, drv:2474-2520) pre-multiplied by the back projector's
+  // segment weight (sbrt:1637-1649); kBatch planes' loads go out together
+  auto finish = [&](auto count, int n, auto plane_of, auto val) {
+    constexpr int kCount = decltype(count)::value, kBatch = 6;
+    const size_t q0 = 2 * ((size_t)x * g.pplanes + g.poff[sg]) + (tid & 1);  // lane pairs
+    const int fs = fr.map ? __ldg(fr.map + frame) : frame;
+    const size_t i0 = (size_t)fs * (fr.input / 2) + 2 * (size_t)w.view * g.nquads * g.pplanes + q0;
+    float2 *o2 = reinterpret_cast<float2 *>(out + (size_t)frame * (fr.ratio / 4) + (size_t)w.slot * out_pair_stride) + q0;
+    const float bs = MODE == 1 ? g.bp_scale[sg] : 0.f;
+    const float *rescale = g.rescale + (gg < 0 ? 0 : gg * g.nz + ybot);
 #pragma unroll
-    for (int j = 0; j < PL; j++) acc[j] = ldq(cen + min(zb + j, ZS - 1));
-  }
-  const int gg = (tk.seg + 1) / 2 - 1;
-  const bool odd = tk.seg & 1;  // segment 2k-1: pam2 at z, pam at z2
-  const int pofs = tk.p0 - g.zshift;
-  const int gs = gg < 0 ? 0 : gg;
-  const int ns_t = (tk.type < 0) ? 0 : g.ytop[tk.seg] - g.ybot[tk.seg] + 1;
-  const int li0 = gg * 2 * g.zshift + ((tk.p0 < g.zshift) ? tk.p0 : tk.p0 - ns_t + 2 * g.zshift);
-  const int FS = g.groupmax * 2 * g.zshift;
-  for (int r = 0; r < nrows; r++) {
-    const int sl = r % kFpSlots, es = r % (2 * kFpSlots), y = ystart + r;
-    bar_sync(kBarFull + sl, nthr);
-    const float4 *pam = rows + (size_t)sl * 2 * ZS;
-    const float4 *pam2 = pam + ZS;
-    if (tk.type == 0) {
-      // theta = 0 (sbrt:1907-1910)
+    for (int j0 = 0; j0 < kCount; j0 += kBatch) {
+      float sc[kBatch];
+      float2 num[kBatch], ad[kBatch];
 #pragma unroll
-      for (int j = 0; j < PL; j++) acc[j] = qadd(acc[j], qadd(ldq(pam + tk.p0 + j), ldq(pam2 + tk.p0 + j)));
-    } else if (tk.type > 0) {
-      const FpMid m = s_mid[es][gs];
-      if (m.z >= 0) {  // else the group is skipped for this row (sbrt:1923-1924)
-        // segment 2k accumulates pam at z and pam2 at z2; segment 2k-1 the converse
-        const float4 *A = odd ? pam2 : pam;
-        const float4 *B = odd ? pam : pam2;
-        if (tk.type == 1) {
-          // middle planes: z, z2 advance with the plane (sbrt:1933-1947)
-          const float4 *Aw = A + m.z + pofs, *Bw = B + m.z2 + pofs;
-          const uint64_t f = pk(m.f, m.f), f2 = pk(m.f2, m.f2);
-          Q2 a0 = ldq(Aw), b0 = ldq(Bw);
+      for (int k = 0; k < kBatch; k++) {
+        if (j0 + k >= kCount) continue;
+        const int p = plane_of(j0 + k < n ? j0 + k : 0);
+        sc[k] = (sg == 0) ? g.y_size : rescale[p];
+        if (MODE == 1) {
+          num[k] = load_p2(prompts, i0 + 2 * p);
+          ad[k] = load_p2(add, i0 + 2 * p);
+        }
+      }
 #pragma unroll
-          for (int j = 0; j < PL; j++) {
-            const Q2 a1 = ldq(Aw + j + 1), b1 = ldq(Bw + j + 1);
-            acc[j] = qadd(acc[j], qaddp(qmul(qadd(b1, a0), f2), qmul(qadd(a1, b0), f), one));
-            a0 = a1;
-            b0 = b1;
-          }
-        } else {
-          // end planes: per-plane flookup entries (sbrt:1925-1931, :1948-1952)
-          const int2 *fy = g.fl_zf + y * FS + li0, *fm = g.fl_zf + (N - y) * FS + li0;
+      for (int k = 0; k < kBatch; k++) {
+        if (j0 + k >= kCount) continue;
+        float2 est = upk(mul2(val(j0 + k), pk(sc[k], sc[k])));
+        if (MODE == 1) {
+          const float d0 = est.x + ad[k].x, d1 = est.y + ad[k].y;
+          const float r0 = num[k].x == 0.f ? 0.f : d0 > g.eps3 ? num[k].x / d0 : 1.0f;
+          const float r1 = num[k].y == 0.f ? 0.f : d1 > g.eps3 ? num[k].y / d1 : 1.0f;
+          est = make_float2(r0 * bs, r1 * bs);
+        }
+        if (j0 + k < n) o2[2 * plane_of(j0 + k)] = est;
+      }
+    }
+  };
+  if (!mbar_wait(&s_cen, 0, g.err)) return;
+  if (kind == 2) {
+    // end planes: per-plane flookup entries (sbrt:1925-1931, :1948-1952), the
+    // next row's in flight under this one's; entry i is plane i (bottom) or
+    // ns - 2*zshift + i (top)
+    auto plane = [&](int i) { return i >= g.zshift ? ns - 2 * g.zshift + i : i; };
+    const int n = tk.type == 2 ? tk.n : 0, FS = G * 2 * g.zshift;
+    const int2 *fl = g.fl_zf + (n ? gg * 2 * g.zshift + tk.p0 : 0);
+    uint64_t acc[kFpEndPlanes];
+    int2 n1[kFpEndPlanes], n2[kFpEndPlanes];
 #pragma unroll
-          for (int j = 0; j < kFpEndPlanes; j++) {
-            if (j < tk.n) {
-              const int2 e1 = __ldg(fy + j), e2 = __ldg(fm + j);
-              const int z = e1.x, z2 = e2.x;
-              const float f = __int_as_float(e1.y), f2 = __int_as_float(e2.y);
-              const uint64_t ff = pk(f, f), ff2 = pk(f2, f2);
-              acc[j] = qadd(acc[j], qaddp(qmul(qadd(ldq(B + z2 + 1), ldq(A + z)), ff2),
-                                          qmul(qadd(ldq(A + z + 1), ldq(B + z2)), ff), one));
-            }
+    for (int j = 0; j < kFpEndPlanes; j++) {
+      acc[j] = centre(plane(tk.p0 + j));
+      n1[j] = n2[j] = make_int2(0, 0);
+    }
+    auto entries = [&](int y) {
+#pragma unroll
+      for (int j = 0; j < kFpEndPlanes; j++)
+        if (j < n) {
+          n1[j] = __ldg(fl + y * FS + j);
+          n2[j] = __ldg(fl + (N - y) * FS + j);
+        }
+    };
+    if (nrows > 0) entries(ystart);
+    for (int r = 0; r < nrows; r++) {
+      int2 e1[kFpEndPlanes], e2[kFpEndPlanes];
+#pragma unroll
+      for (int j = 0; j < kFpEndPlanes; j++) {
+        e1[j] = n1[j];
+        e2[j] = n2[j];
+      }
+      if (r + 1 < nrows) entries(ystart + r + 1);
+      if (!next_row(r)) return;
+      const int sl = r & (kFpSlots - 1), at = sl * row_bytes;
+      if (mid[sl * G].z >= 0) {
+#pragma unroll
+        for (int j = 0; j < kFpEndPlanes; j++) {
+          if (j < n) {
+            const int pa = at + oA + 16 * e1[j].x, pb = at + oB + 16 * e2[j].x;
+            const float f = __int_as_float(e1[j].y), f2 = __int_as_float(e2[j].y);
+            const uint64_t ff = pk(f, f), ff2 = pk(f2, f2);
+            acc[j] = add2(acc[j], addp(mul2(add2(lds2(smem, pb + 16), lds2(smem, pa)), ff2),
+                                       mul2(add2(lds2(smem, pa + 16), lds2(smem, pb)), ff), one));
           }
         }
       }
+      row_done(r);
     }
-    if (r + kFpSlots < nrows) bar_arrive(kBarEmpty + sl, nthr);
+    if (n) finish(std::integral_constant<int, kFpEndPlanes>{}, n, [&](int j) { return plane(tk.p0 + j); },
+                  [&](int j) { return acc[j]; });
+    return;
   }
-
-  // scale (sbrt:1953-1975), then either store the estimate or the OP ratio
-  // (pt_update_est_w3, drv:2474-2520) pre-multiplied by the back projector's
-  // segment weight (sbrt:1637-1649)
-  if (tk.type < 0) return;
-  const size_t qbase = (size_t)x * g.pplanes;
-  const int sg = tk.seg;
+  uint64_t acc[PL];
 #pragma unroll
-  for (int j = 0; j < PL; j++) {
-    if (j >= tk.n) continue;
-    const int r = tk.p0 + j, yr = g.ybot[sg] + r;
-    const float sc = (sg == 0) ? g.y_size : g.rescale[gg * g.nz + yr];
-    const float4 est = q2f(qmul(acc[j], pk(sc, sc)));
-    const size_t qi = qbase + g.poff[sg] + r;
-    if (MODE == 0) {
-      out[(size_t)w.slot * out_pair_stride + qi] = est;
-    } else {
-      const size_t ii = (size_t)v * g.nquads * g.pplanes + qi;
-      const P4 p = load_p4(prompts, ii);
-      const P4 ad = load_p4(add, ii);
-      const float bs = g.bp_scale[sg];
-      float rr[4];
+  for (int j = 0; j < PL; j++) acc[j] = centre(tk.p0 + j);
+  if (kind == 1) {
+    // middle planes: z, z2 advance with the plane (sbrt:1933-1947)
+    const int o = 16 * (tk.p0 - g.zshift);
+    for (int r = 0; r < nrows; r++) {
+      if (!next_row(r)) return;
+      const int sl = r & (kFpSlots - 1);
+      const FpMid m = mid[sl * G];
+      if (tk.type == 1 && m.z >= 0) {  // else the group is skipped for this row (sbrt:1923-1924)
+        const int at = sl * row_bytes + o, pa = at + oA + 16 * m.z, pb = at + oB + 16 * m.z2;
+        const uint64_t f = pk(m.f, m.f), f2 = pk(m.f2, m.f2);
+        uint64_t a0 = lds2(smem, pa), b0 = lds2(smem, pb);
 #pragma unroll
-      for (int l = 0; l < 4; l++) {
-        const float den = lane(est, l) + ad.v[l];
-        float q;
-        if (p.v[l] == 0.f) q = 0.f;
-        else if (den > g.eps3) q = p.v[l] / den;
-        else q = 1.0f;
-        rr[l] = q * bs;
+        for (int j = 0; j < PL; j++) {
+          const uint64_t a1 = lds2(smem, pa + 16 * (j + 1)), b1 = lds2(smem, pb + 16 * (j + 1));
+          acc[j] = add2(acc[j], addp(mul2(add2(b1, a0), f2), mul2(add2(a1, b0), f), one));
+          a0 = a1;
+          b0 = b1;
+        }
       }
-      out[(size_t)w.slot * out_pair_stride + qi] = make_float4(rr[0], rr[1], rr[2], rr[3]);
+      row_done(r);
+    }
+  } else {
+    // theta = 0 (sbrt:1907-1910)
+    for (int r = 0; r < nrows; r++) {
+      if (!next_row(r)) return;
+      const int at = (r & (kFpSlots - 1)) * row_bytes + 16 * tk.p0 + q8;
+#pragma unroll
+      for (int j = 0; j < PL; j++)
+        acc[j] = add2(acc[j], add2(lds2(smem, at + 16 * j), lds2(smem, at + 16 * ZS + 16 * j)));
+      row_done(r);
     }
   }
+  if (tk.type < 0) return;
+  finish(std::integral_constant<int, PL>{}, tk.n, [&](int j) { return tk.p0 + j; }, [&](int j) { return acc[j]; });
 }
 
 // ============================================================================
@@ -1426,106 +1402,63 @@ __global__ void scale_pairs_kernel(DevGeom g, const T *__restrict__ src, const i
   dst[(size_t)slot * dst_pair_stride + i] = o;
 }
 
-// The images the forward projector samples as a 4-D tensor (z, y, x, stored
-// frame) with a box of the four corner columns of one sample point, {zp, 2,
-// 2, 1}: one bulk tensor copy instead of two per point (the projector's row
-// pipeline is bound by the number of copies, not their bytes).  Returns 0 (the
-// kernel then copies column pairs) where the encoder is unavailable or
-// refuses the shape.
-using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-int image_column_map(const DevGeom &g, const float *image, const FrameStrides &fr, CUtensorMap *map) {
-  static EncodeTiledFn encode = [] {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess) {
-      cudaGetLastError();
-      return (EncodeTiledFn) nullptr;
-    }
-    return reinterpret_cast<EncodeTiledFn>(fn);
-  }();
-  std::memset(map, 0, sizeof(*map));
-  if (!encode || !image || (reinterpret_cast<uintptr_t>(image) & 15)) return 0;
-  const cuuint64_t N = (cuuint64_t)g.nx, zp = (cuuint64_t)g.zp;
-  const cuuint64_t fstride = fr.image > 0 ? (cuuint64_t)fr.image : N * N * zp;
-  // stored frames: every frame a launch may name (the map bounds no access the
-  // kernel makes; coordinates stay inside the frames that exist)
-  const cuuint64_t frames = fr.image > 0 ? (cuuint64_t)1 << 16 : 1;
-  const cuuint64_t dim[4] = {zp, N, N, frames};
-  const cuuint64_t stride[3] = {zp * 4, N * zp * 4, fstride * 4};
-  const cuuint32_t box[4] = {(cuuint32_t)zp, 2, 2, 1};
-  const cuuint32_t es[4] = {1, 1, 1, 1};
-  if (zp > 256 || (zp * 4) % 16 || (fstride * 4) % 16) return 0;
-  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(image), dim, stride, box, es,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 1 : 0;
-}
-
-template <int MODE, int PL, int MW, typename PT, typename AT>
-cudaError_t launch_fp_t(const DevGeom &g, const float *image, const QuadWork *work, int nwork, const void *prompts,
-                        const void *add, float *out, long long out_pair_stride, int pwarps_req,
-                        const FrameStrides &fr, cudaStream_t st) {
-  // consumer warps: one task per thread; producer warps: enough to keep the
-  // sampled rows ahead of the consumers (a row is ~2*zp bilinear quads)
-  const int cwarps = (g.nfptasks + 31) / 32;
-  const int pwarps = pwarps_req > 0 ? pwarps_req : min(6, max(2, MW - cwarps));
-  if (pwarps < 2 || cwarps + pwarps > MW) return cudaErrorInvalidConfiguration;
-  const int threads = (cwarps + pwarps) * 32;
+template <int MODE, int PL, typename PT, typename AT>
+cudaError_t launch_fp_t(const DevGeom &g, const float *samples, const QuadWork *work, int nwork, const void *prompts,
+                        const void *add, float *out, long long out_pair_stride, const FrameStrides &fr,
+                        cudaStream_t st) {
+  const int warps = g.nfptasks / 16 + 1;
   const int ZS = g.zp + kFpZPad;
-  const size_t smem =
-      (size_t)(kFpSlots * 8 * 2 + 2) * 2 * g.zp * sizeof(float) + (size_t)(2 * kFpSlots + 1) * ZS * sizeof(float4);
-  auto k = fp_kernel<MODE, PL, MW, PT, AT>;
+  const size_t smem = (size_t)(2 * kFpSlots + 1) * ZS * sizeof(float4) + (size_t)kFpSlots * g.groupmax * sizeof(FpMid);
+  auto k = fp_kernel<MODE, PL, PT, AT>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  CUtensorMap cols;
-  const int use_cols = image_column_map(g, image, fr, &cols);
-  k<<<(unsigned)nwork * fr.n, threads, smem, st>>>(g, image, work, (const PT *)prompts, (const AT *)add,
-                                                   reinterpret_cast<float4 *>(out), out_pair_stride / 4, pwarps, fr,
-                                                   cols, use_cols);
+  k<<<(unsigned)nwork * fr.n, warps * 32, smem, st>>>(g, reinterpret_cast<const float4 *>(samples), work,
+                                                      (const PT *)prompts, (const AT *)add,
+                                                      reinterpret_cast<float4 *>(out), out_pair_stride / 4, fr);
   return cudaGetLastError();
 }
 
-template <int PL, int MW>
-cudaError_t launch_fp_pl(const DevGeom &g, const float *image, const QuadWork *work, int nwork, int mode,
-                         const void *prompts, const void *add, int storage, float *out, long long stride, int pwarps,
+template <int PL>
+cudaError_t launch_fp_pl(const DevGeom &g, const float *samples, const QuadWork *work, int nwork, int mode,
+                         const void *prompts, const void *add, int storage, float *out, long long stride,
                          const FrameStrides &fr, cudaStream_t st) {
   if (mode == 0)
-    return launch_fp_t<0, PL, MW, int16_t, float>(g, image, work, nwork, nullptr, nullptr, out, stride, pwarps, fr,
-                                                  st);
+    return launch_fp_t<0, PL, int16_t, float>(g, samples, work, nwork, nullptr, nullptr, out, stride, fr, st);
   if (storage == 0)
-    return launch_fp_t<1, PL, MW, int16_t, float>(g, image, work, nwork, prompts, add, out, stride, pwarps, fr, st);
+    return launch_fp_t<1, PL, int16_t, float>(g, samples, work, nwork, prompts, add, out, stride, fr, st);
   if (storage == 1)
-    return launch_fp_t<1, PL, MW, int16_t, __nv_bfloat16>(g, image, work, nwork, prompts, add, out, stride, pwarps,
-                                                          fr, st);
-  return launch_fp_t<1, PL, MW, int16_t, __half>(g, image, work, nwork, prompts, add, out, stride, pwarps, fr, st);
+    return launch_fp_t<1, PL, int16_t, __nv_bfloat16>(g, samples, work, nwork, prompts, add, out, stride, fr,
+                                                      st);
+  return launch_fp_t<1, PL, int16_t, __half>(g, samples, work, nwork, prompts, add, out, stride, fr, st);
 }
 
 }  // namespace
 
-cudaError_t launch_fp(const DevGeom &g, const float *image, const QuadWork *work, int nwork, int mode,
-                      const void *prompts, const void *add, int storage, float *out, long long out_pair_stride,
-                      const ProjTune &tune, const FrameStrides &fr, cudaStream_t st) {
+cudaError_t launch_fp(const DevGeom &g, const float *image, float *samples, const int *pair_views, int view0,
+                      int npairs, const QuadWork *work, int nwork, int mode, const void *prompts, const void *add,
+                      int storage, float *out, long long out_pair_stride, const FrameStrides &fr, cudaStream_t st) {
   if (nwork <= 0 || fr.n <= 0) return cudaSuccess;
-  static_assert(kFpPlaneVariants[0] == 7 && kFpPlaneVariants[1] == 9 && kFpPlaneVariants[2] == 11, "variants");
-  const int pl = tune.fp_planes > 0 ? tune.fp_planes : kFpPlanes;
-  switch (pl) {
-    case 7:
-      return launch_fp_pl<7, kFpVariantWarps[0]>(g, image, work, nwork, mode, prompts, add, storage, out,
-                                                 out_pair_stride, tune.fp_pwarps, fr, st);
-    case 9:
-      return launch_fp_pl<9, kFpVariantWarps[1]>(g, image, work, nwork, mode, prompts, add, storage, out,
-                                                 out_pair_stride, tune.fp_pwarps, fr, st);
-    case 11:
-      return launch_fp_pl<11, kFpVariantWarps[2]>(g, image, work, nwork, mode, prompts, add, storage, out,
-                                                  out_pair_stride, tune.fp_pwarps, fr, st);
-    default:
-      return cudaErrorInvalidValue;
+  constexpr int T = kSampleTile;
+  // the frames go in turns where they would exceed the grid's third dimension
+  for (int f0 = 0, per = 65535 / (2 * npairs); f0 < fr.n; f0 += per) {
+    FrameStrides part = fr;
+    part.n = std::min(per, fr.n - f0);
+    if (fr.map) part.map = fr.map + f0;
+    // 8 rows a warp, fewer where that leaves SMs without their two CTAs
+    const int nx = (g.c + T - 1) / T, nz = 2 * npairs * part.n;
+    int steps = 16;
+    while (steps > 1 && (long long)nx * nz * (g.c / (T * steps) + 1) < 8 * 148) steps /= 2;
+    fp_sample_kernel<<<dim3(nx, g.c / (T * steps) + 1, nz), T * T * 32, 0, st>>>(
+        g, image + (fr.map ? 0 : (size_t)f0 * fr.image), pair_views, view0, npairs,
+        reinterpret_cast<float4 *>(samples + (size_t)f0 * fr.samples), part, steps);
   }
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  auto f = g.fp_run == kFpRuns[0]   ? launch_fp_pl<kFpRuns[0]>
+           : g.fp_run == kFpRuns[1] ? launch_fp_pl<kFpRuns[1]>
+           : g.fp_run == kFpRuns[2] ? launch_fp_pl<kFpRuns[2]>
+                                    : launch_fp_pl<kFpRuns[3]>;
+  return f(g, samples, work, nwork, mode, prompts, add, storage, out, out_pair_stride, fr, st);
 }
 
 template <bool ACC, bool MULTI>

@@ -23,13 +23,10 @@
 
 namespace hrrt {
 
-#ifndef HRRT_FP_SLOTS
-#define HRRT_FP_SLOTS 3
-#endif
-constexpr int kFpPlanes = 9;                   // default planes per forward-projection task (odd: bank-conflict free)
-constexpr int kFpSlots = HRRT_FP_SLOTS;       // sampled rows in flight between producers and consumers
-constexpr int kFpZPad = 16;     // zeroed entries after each sampled row
-constexpr int kFpEndPlanes = 4; // planes per end-plane task (they cost ~2x a middle plane)
+constexpr int kFpPlanes = 9;                   // default plane variant of the forward projector (kFpPlaneVariants)
+constexpr int kFpSlots = 8;     // sampled rows in flight to the forward projector's consumers (a power of 2)
+constexpr int kFpZPad = 44;     // zeroed entries after each sampled row (rows are then 4 modulo 8 entries long)
+constexpr int kFpEndPlanes = 4; // entries per end-plane task
 constexpr int kFpMaxGroups = 32; // segment groups the forward projector stages per row (22 at span 3)
 constexpr int kBpZ = 4;         // z per back-projection task
 constexpr int kBpRows = 4;      // rotated rows per back-projection task (rows kBpRows*m .. kBpRows*m+3)
@@ -37,11 +34,14 @@ constexpr int kAdjZ = 8;        // z per task of the exact adjoint
 constexpr int kBpPad = 8;       // zero planes on each side of a segment in the back projector
 constexpr int kAdjCover = 8;    // rotated-frame points whose bilinear footprint covers a voxel (at most 5 on HRRT)
 
+// A forward-projection task, shared by two threads (lanes 0,1 and 2,3 of the
+// quad).  Types 0 and 1: planes p0 .. p0+n-1 relative to the segment's
+// yr_bottom; type 2: entries p0 .. p0+n-1 of the segment's 2*zshift end planes
+// (bottom ones, then top ones), as the end-plane tables list them.
 struct FpTask {
   int16_t seg;   // segment (internal = file order)
-  int16_t p0;    // first plane, relative to the segment's yr_bottom
-  int16_t n;     // planes in this task (<= the launch's plane variant)
-  int16_t type;  // 0: segment 0, 1: oblique middle planes, 2: oblique end planes
+  int16_t p0, n;
+  int16_t type;  // 0: segment 0, 1: oblique middle planes, 2: oblique end planes, -1: none
 };
 
 struct FpMid {   // middle-plane sampling of group g at rotated row y < c (sbrt:1933-1947)
@@ -77,6 +77,7 @@ struct DevGeom {
   int fov_columns, z_min, z_max;
   float y_size, eps1, eps3, image_max;
   float unit;                       // 1.0f, a run-time value (see addp in kernels.cu)
+  uint64_t unit2;                   // the same as a pair
   const int16_t *cyl0, *cyl1;       // [ny]
   const int *ybot, *ytop, *poff;    // [nseg]; poff = padded offset of plane yr_bottom
   const float *rescale;             // [groupmax][nz]
@@ -96,8 +97,10 @@ struct DevGeom {
   const float *sin_psi, *cos_psi;   // [nviews]
   const short2 *fov_xy;             // [fov_columns]
   const float2 *rotpos;             // [nviews/2][fov_columns] rotate-back sample points
+  const int *samp_off;              // [c + 1] samples of quad x in a pair slot's block (entries of 4 lanes)
+  int samp_pair, samp_rows;         // entries per pair slot; rotated rows of the longest quad
   const FpTask *fptasks;
-  int nfptasks;
+  int nfptasks, fp_run;             // tasks, and planes of the longest (kFpRuns)
   const int16_t *plane_seg;         // [segmentsize] segment of each global plane
   const int16_t *pplane_seg;        // [pplanes] segment of each padded plane, -1 on pads
   int *err;                         // device status word: non-zero after a bounded wait gave up
@@ -132,8 +135,9 @@ struct FrameStrides {
   long long ratio;    // floats between ratio blocks ([pair slot][quad_pair])
   long long bc;       // floats between back-projection partial blocks (Bc and Br alike)
   long long partial;  // doubles between post-iteration partial-sum arrays
+  long long samples;  // floats between the forward projector's sample blocks
 };
-inline FrameStrides one_frame() { return FrameStrides{1, nullptr, 0, 0, 0, 0, 0}; }
+inline FrameStrides one_frame() { return FrameStrides{1, nullptr, 0, 0, 0, 0, 0, 0}; }
 
 // launch shape of the projectors (results do not depend on it)
 struct ProjTune {
@@ -147,16 +151,24 @@ struct ProjTune {
 };
 inline ProjTune default_tune() { return ProjTune{0, 0, 0, 0, 0}; }
 constexpr int kFpPlaneVariants[3] = {7, 9, 11};
-// warps per forward-projection CTA for each plane variant (register budget)
+// Planes per task that the kernel is built for (odd: the runs of a segment
+// start in different bank groups).  Variant i takes the first of runs i.. that
+// leaves room for a producer warp beside the consumers; a variant is offered
+// where one thread per (segment, kFpPlaneVariants[i] planes) and two producer
+// warps would fit kFpVariantWarps[i] warps.
+constexpr int kFpRuns[4] = {13, 17, 21, 25};
 constexpr int kFpVariantWarps[3] = {32, 32, 24};
+constexpr int kFpMaxWarps = 32;
 
 // ---- launchers (kernels.cu) ----
 // forward projection of the pairs listed in `work` (mode 0: write est*scale into
 // `out`; mode 1: write ratio*bp_scale using prompts/add at their global pair).
-// `g.fptasks` must be the task list built for tune.fp_planes.
-cudaError_t launch_fp(const DevGeom &g, const float *image, const QuadWork *work, int nwork, int mode,
-                      const void *prompts, const void *add, int storage, float *out, long long out_pair_stride,
-                      const ProjTune &tune, const FrameStrides &fr, cudaStream_t st);
+// `g.fptasks` a list of g.fp_run planes a task; `samples` scratch of
+// 4 * g.samp_pair floats for each of the `npairs` pair slots; slot k is view
+// pair_views[k], or view0 + k where that is null.
+cudaError_t launch_fp(const DevGeom &g, const float *image, float *samples, const int *pair_views, int view0,
+                      int npairs, const QuadWork *work, int nwork, int mode, const void *prompts, const void *add,
+                      int storage, float *out, long long out_pair_stride, const FrameStrides &fr, cudaStream_t st);
 // back projection of quad-layout input into the column (Bc) / row (Br) partials
 cudaError_t launch_bp(const DevGeom &g, const float *in, long long in_pair_stride, const QuadWork *work, int nwork,
                       float *bc, float *br, long long vol, const FrameStrides &fr, cudaStream_t st);

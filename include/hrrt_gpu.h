@@ -311,7 +311,8 @@ typedef struct hrrt_batch_stats {
   int groups;             /* frame groups (launches cover one group) */
   int graphs;             /* CUDA graphs captured */
   int graph_launches;     /* graph replays (one per iteration of a group) */
-  long long kernel_launches; /* kernels run by those replays */
+  long long kernel_launches; /* phases launched by those replays: forward projection (its two kernels count once),
+                                back projection and update of each subset, and the two of the post-iteration pass */
 } hrrt_batch_stats;
 
 /* norm / atten: flat-file arrays shared by every frame (NULL = 1), copied to
