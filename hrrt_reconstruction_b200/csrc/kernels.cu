@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(kFpMaxWarps * 32, 1) fp_kernel(DevGeom g, cons
 // the segment less than a plane apart, so four rows share a window -- and
 // issues 50 packed FMAs and about 65 other instructions.  One row and 8
 // planes a thread (9 shared planes for 8 outputs, an address each) took
-// 1.384 ms a span-3 subset and 0.509 ms a span-9 one; this 0.892 and 0.361.
+// 1.384 ms a span-3 subset and 0.509 ms a span-9 one; this 0.892 and 0.343.
 // Measured and not used: the row pattern as arithmetic instead of a branch (both
 // slopes applied, one of them 0: 1.021 ms), lane pairs split over two threads
 // for twice the warps (0.941 ms), no prefetch of the next entry (0.977 ms).
@@ -805,7 +805,13 @@ __global__ void __launch_bounds__(kBpThreads<ACC>, 2) bp_kernel(DevGeom g, const
 // the middle planes are two windows of the segment, the end planes one
 // position each), with the rows first scaled as the forward projector scales
 // them (sbrt:1953-1976).  The samples are the back projector's voxel roles, so
-// the lanes go to the same column / row partials.
+// the lanes go to the same column / row partials.  An output plane gathers
+// its end planes by table (at most four consecutive ones; a geometry where
+// it takes more walks the entries in order instead: GATHER false).  Bound by
+// the shared reads and the chain of table -> end plane -> FMA: four planes'
+// entries in flight at three CTAs an SM measured 1057 us a span-9 subset of
+// the HRRT (1329 entry by entry; one plane at a time 1322, eight planes at
+// two CTAs 1315, two at four 1621); without any end planes 560.
 // adj_rotate_kernel: the bilinear sampling transposed as a gather: an image
 // voxel collects from the <= 16 rotated-frame points around its inverse
 // rotation whose sample footprint (recomputed with the forward projector's own
@@ -840,7 +846,8 @@ __device__ __forceinline__ void adj_side(Q2 (&s)[KB], const float4 *__restrict__
   }
 }
 
-template <int KB>
+constexpr int kAdjBatch = 4;
+template <int KB, bool GATHER>
 __global__ void __launch_bounds__(256, 3) adj_kernel(DevGeom g, const float4 *__restrict__ in, long long in_pair_stride,
                                                   const QuadWork *__restrict__ work, float *__restrict__ bc,
                                                   float *__restrict__ br, long long vol, FrameStrides fr) {
@@ -917,6 +924,43 @@ __global__ void __launch_bounds__(256, 3) adj_kernel(DevGeom g, const float4 *__
           const uint64_t f = pk(m.f, m.f), f2 = pk(m.f2, m.f2);
           adj_side<KB>(s, A, z0 - m.z + ym, ym, ye, f2, f);
           adj_side<KB>(s, B, z0 - m.z2 + ym, ym, ye, f, f2);
+          if (GATHER) {
+            // end planes: what each output plane takes from them, by table
+#pragma unroll 1
+            for (int k = 0; k < 4; k++) {  // side k / 2, end k & 1
+              const size_t zb = ((size_t)gg * 4 + k) * c + y;
+              const short2 zr = __ldg(g.adj_endz + zb);
+              if (z0 > zr.y || z0 + KB - 1 < zr.x) continue;
+              const float4 *E = (k < 2 ? A : B) + ((k & 1) ? yt - ZS + 1 : yb);
+              const size_t tb = ((size_t)gg * 4 + k) * kAdjEndOut * c + y;
+#pragma unroll
+              for (int j0 = 0; j0 < KB; j0 += kAdjBatch) {
+                // kAdjBatch planes' entries in flight together
+                int en[kAdjBatch];
+                float4 wt[kAdjBatch];
+#pragma unroll
+                for (int i = 0; i < kAdjBatch; i++) {
+                  const int z = z0 + j0 + i;
+                  const bool in = z >= zr.x && z <= zr.y;
+                  const size_t at = tb + (size_t)(in ? z - zr.x : 0) * c;
+                  en[i] = __ldg(reinterpret_cast<const int *>(g.adj_ends) + at);
+                  wt[i] = __ldg(g.adj_endw + at);
+                  if (!in) en[i] = 0;
+                }
+#pragma unroll
+                for (int i = 0; i < kAdjBatch; i++) {
+                  const float4 *e0 = E + (int)(int16_t)(en[i] & 0xffff);
+                  const int n = en[i] >> 16;
+                  Q2 &t = s[j0 + i];
+                  if (n > 0) t = qfma(ldq(e0), pk(wt[i].x, wt[i].x), t);
+                  if (n > 1) t = qfma(ldq(e0 + 1), pk(wt[i].y, wt[i].y), t);
+                  if (n > 2) t = qfma(ldq(e0 + 2), pk(wt[i].z, wt[i].z), t);
+                  if (n > 3) t = qfma(ldq(e0 + 3), pk(wt[i].w, wt[i].w), t);
+                }
+              }
+            }
+            continue;
+          }
           // end planes: one position per plane; an end whose entries touch
           // no plane of this task's run is skipped whole
           const size_t eb = (size_t)gg * 2 * ZS * N;
@@ -1402,6 +1446,21 @@ __global__ void scale_pairs_kernel(DevGeom g, const T *__restrict__ src, const i
   dst[(size_t)slot * dst_pair_stride + i] = o;
 }
 
+// Dynamic shared memory of a kernel that has `ctas` CTAs resident per SM by its
+// registers; what they leave of the SM's memory stays L1, which holds the
+// sampling tables the projectors read (the whole SM's memory as shared memory
+// instead: adjoint 1200 us a subset at span 9 against 1057, back projector 361
+// against 343).
+template <typename K>
+cudaError_t set_smem(K k, size_t smem, int ctas) {
+  constexpr size_t kSm = 228 * 1024, kReserved = 1024;  // of an SM; of a CTA
+  ctas = (int)std::max<size_t>(1, std::min<size_t>(ctas, kSm / (smem + kReserved)));
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int pct = (int)std::min<size_t>(100, (ctas * (smem + kReserved) * 100 + kSm - 1) / kSm);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+  return e;
+}
+
 template <int MODE, int PL, typename PT, typename AT>
 cudaError_t launch_fp_t(const DevGeom &g, const float *samples, const QuadWork *work, int nwork, const void *prompts,
                         const void *add, float *out, long long out_pair_stride, const FrameStrides &fr,
@@ -1410,7 +1469,7 @@ cudaError_t launch_fp_t(const DevGeom &g, const float *samples, const QuadWork *
   const int ZS = g.zp + kFpZPad;
   const size_t smem = (size_t)(2 * kFpSlots + 1) * ZS * sizeof(float4) + (size_t)kFpSlots * g.groupmax * sizeof(FpMid);
   auto k = fp_kernel<MODE, PL, PT, AT>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = set_smem(k, smem, std::max(1, 32 / warps));
   if (e != cudaSuccess) return e;
   k<<<(unsigned)nwork * fr.n, warps * 32, smem, st>>>(g, reinterpret_cast<const float4 *>(samples), work,
                                                       (const PT *)prompts, (const AT *)add,
@@ -1467,9 +1526,7 @@ cudaError_t launch_bp_t(const DevGeom &g, const float *in, long long in_pair_str
                         cudaStream_t st) {
   const size_t smem = (size_t)4 * g.bp_s4 * sizeof(float4);
   auto k = bp_kernel<ACC, MULTI>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  cudaError_t e = set_smem(k, smem, 2);
   if (e != cudaSuccess) return e;
   // launches that do not fill the chip share each quad among several CTAs
   const long long quads = (long long)nquads * fr.n;
@@ -1490,10 +1547,8 @@ cudaError_t launch_adj(const DevGeom &g, const float *in, long long in_pair_stri
                        float *bc, float *br, long long vol, const FrameStrides &fr, cudaStream_t st) {
   if (nwork <= 0 || fr.n <= 0) return cudaSuccess;
   const size_t smem = (size_t)g.bp_splanes * sizeof(float4);
-  auto k = adj_kernel<kAdjZ>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  auto k = g.adj_ends ? adj_kernel<kAdjZ, true> : adj_kernel<kAdjZ, false>;
+  cudaError_t e = set_smem(k, smem, 3);
   if (e != cudaSuccess) return e;
   k<<<(unsigned)nwork * fr.n, 256, smem, st>>>(g, reinterpret_cast<const float4 *>(in), in_pair_stride / 4, work, bc,
                                                br, vol, fr);

@@ -56,6 +56,17 @@ struct BpLut {   // blookup (sbrt:672-700) in direct form: yr = z + d for z in [
   float f;
 };
 
+// The exact adjoint's end planes as a gather: output plane zs + k takes the
+// `n` consecutive end planes from i0 on (of the zshift at that end) with the
+// weights w; adj_ends holds [groupmax][2 sides][2 ends][kAdjEndOut][c] of
+// them, adj_endz the ranges (first, last output plane) [groupmax][2][2][c].
+// Side 0 are the rows that read a sample at the row's own positions, side 1
+// those that read it at its mirror's.
+constexpr int kAdjEndOut = 24;
+struct AdjEnd {
+  int16_t i0, n;
+};
+
 // One side of a segment group in the back projection of a row group: the rows
 // read the segment at yr = z + shift with a fraction f (BpLut), and the shifts
 // of adjacent rows differ by less than one plane, so that the four rows share
@@ -88,6 +99,9 @@ struct DevGeom {
   const int2 *fl_t;                 // fl_zf transposed: [groupmax*2*zshift][ny]
   const int4 *adj_endr;             // exact adjoint, [groupmax][c]: planes the bottom / top end-plane
                                     //   entries of a row touch (x..y bottom, z..w top; empty: lo > hi)
+  const AdjEnd *adj_ends;           // null where the end planes do not gather (AdjEnd): entry by entry then
+  const float4 *adj_endw;           //   the weights of each of these
+  const short2 *adj_endz;
   int2 *adj_ent;                    // exact adjoint's rotate: per (pair slot, column) the covering
   int *adj_cnt;                     //   rotated-frame points (index, weight bits) [.][kAdjCover], their count
   int adj_pairs;                    //   pair slots the two buffers hold (for every image column)
