@@ -806,8 +806,9 @@ __global__ void __launch_bounds__(kBpThreads<ACC>, 2) bp_kernel(DevGeom g, const
 // position each), with the rows first scaled as the forward projector scales
 // them (sbrt:1953-1976).  The samples are the back projector's voxel roles, so
 // the lanes go to the same column / row partials.  An output plane gathers
-// its end planes by table (at most four consecutive ones; a geometry where
-// it takes more walks the entries in order instead: GATHER false).  Bound by
+// its end planes by table (at most four consecutive ones); where it takes
+// more, or an end has few planes, the task walks the entries in order (GATHER
+// false).  Bound by
 // the shared reads and the chain of table -> end plane -> FMA: four planes'
 // entries in flight at three CTAs an SM measured 1057 us a span-9 subset of
 // the HRRT (1329 entry by entry; one plane at a time 1322, eight planes at

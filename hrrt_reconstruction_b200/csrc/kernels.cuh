@@ -63,6 +63,7 @@ struct BpLut {   // blookup (sbrt:672-700) in direct form: yr = z + d for z in [
 // Side 0 are the rows that read a sample at the row's own positions, side 1
 // those that read it at its mirror's.
 constexpr int kAdjEndOut = 24;
+constexpr int kAdjGatherShift = 6;  // end planes an end from which the table pays
 struct AdjEnd {
   int16_t i0, n;
 };

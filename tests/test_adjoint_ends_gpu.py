@@ -9,20 +9,24 @@ from geoms import product_geom, random_rows
 pytestmark = pytest.mark.gpu
 
 BASE = dict(plane_sep=1.21875, binsize=1.21875, subsets=16)
-# name -> (geometry, whether every output plane takes at most four end planes)
+# name -> (geometry, whether its end planes gather by table)
 GEOMS = {
     "ragged9": (dict(BASE, nrings=59, nelements=148, nangles=160, ring_radius=134.5, span=9, maxdel=38, subsets=10), True),
-    "ragged3": (dict(BASE, nrings=27, nelements=68, nangles=96, ring_radius=62.0, span=3, maxdel=16), True),
+    "ragged3": (dict(BASE, nrings=27, nelements=68, nangles=96, ring_radius=62.0, span=3, maxdel=16), False),
+    "ragged7": (dict(BASE, nrings=28, nelements=68, nangles=96, ring_radius=62.0, span=7, maxdel=17), True),
     "steep9": (dict(BASE, nrings=32, nelements=64, nangles=96, ring_radius=34.0, span=9, maxdel=22), False),
 }
 
 
 def gathers(d):
-    """At most 4 consecutive end planes reach an output plane, and no end's
-    outputs span 24 planes (rows 1 .. c-1 and their mirrors)."""
+    """At least 6 end planes an end, of which at most 4 consecutive ones reach
+    an output plane, and no end's outputs span 24 planes (rows 1 .. c-1 and
+    their mirrors)."""
     import hrrt_reconstruction_b200 as H
     zi = H.geometry_table(product_geom(d), "flookup_zzi")
     zs, N = d["span"] - 1, d["nelements"]
+    if zs < 6:
+        return False
     zi = zi.reshape(N, -1, 2, zs)
     rows = zi[[y for y in range(1, N) if y != N // 2]].reshape(-1, zs)
     for r in rows:
