@@ -7,20 +7,19 @@
 // rebins events through a crystal-pair LUT, and increments 16-bit bins in
 // stream order until a time tag ends the frame.
 //
-// Device design.  The word stream is cut into tiles of kTileWords words (a
-// tile never straddles a packet); a block of 256 threads owns a tile, each
-// thread 16 consecutive words.  Where a thread's parse starts depends on the
-// words before it, but only through one bit: whether the previous event
-// ended on the thread's first word or ran one word into it.  Each thread
-// therefore parses its words twice (entering at offset 0 and at offset 1),
-// which yields a 2-state map (entry -> exit) plus the number of time tags
-// seen for each entry.  Maps compose associatively, so
-//   lm_map_kernel   : block scan -> one composed map per tile;
-//   lm_entry_kernel : one thread per packet walks its tiles -> tile entry
-//                     offsets and per-tile time-tag offsets;
+// Device design.  The parse needs no serial walk: a pair of words (a, b) is
+// in sync only when a's top bit is clear and b's is set (kEwTypes), so no two
+// adjacent positions are both in sync, and a position that is in sync is
+// always reached -- the position before it is out of sync, or the second
+// word of the event before it.  Every in-sync pair of a packet is an event,
+// every other position outside an event's second word a resynchronisation.
+// The stream is cut into tiles of kTileWords words (a tile never straddles a
+// packet) of a block each; a thread loads four runs of four words (coalesced
+// 16-byte loads, all in flight) and the word after each from its neighbour:
+//   lm_map_kernel   : time tags per tile (only the tags depend on the order);
+//   lm_entry_kernel : a warp per packet, time-tag offsets of its tiles;
 //   lm_scan_kernel  : exclusive scan of the per-packet tag counts;
-//   lm_hist_kernel  : re-derives each thread's entry with the same block
-//                     scan, parses its words once, writes the time tags in
+//   lm_hist_kernel  : ranks its time tags with ballots, writes them in
 //                     stream order and (below the frame limit) adds the
 //                     events to the sinograms.
 // The frame end is found on the host from the ordered time tags (the clock
@@ -47,8 +46,9 @@
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kSub = 16;                       // words per thread
-constexpr int kTileWords = kThreads * kSub;    // 4096
+constexpr int kRuns = 4;                       // runs of 4 words per thread
+constexpr int kEv = 2 * kRuns;                 // events that start in them at most
+constexpr int kTileWords = kThreads * kRuns * 4;  // 4096
 constexpr long long kPacketWords = 2LL << 20;  // 1 Mi 64-bit events
 static_assert(kPacketWords % kTileWords == 0, "tiles must not straddle packets");
 constexpr int kSinoPlane = 256 * 288;
@@ -56,14 +56,15 @@ constexpr int kSinoPlane = 256 * 288;
 // with atomics whose old value is checked for a carry.  Wide: 32-bit counters
 // updated with reductions that return nothing, folded into the 16-bit bins at
 // the end.  Partitioned: events scattered by 64 MB partition and added
-// partition by partition in L2.  On B200, for 2.5e8 events: direct 14.3 ms,
-// wide 17.0 ms (the random read-modify-write of a DRAM sector per event bounds
-// both; the wide path adds a clear and a fold of 4-byte counters), partitioned
-// 21.0 ms (two extra parses), so the other two run only when asked for.  A
-// fourth way, rebinning every event into a 4-byte record in stream order and
-// adding the records in a separate pass with 30 registers a thread (eight
-// blocks per SM, more adds in flight), measured 19.1 ms: the adds are bound
-// by the DRAM sectors they read and write, not by how many are in flight.
+// partition by partition in L2.  On B200, for 1e8 / 4e8 events: direct 4.8 /
+// 18.9 ms (the random read-modify-write of a DRAM sector per event bounds it),
+// wide 7.0 / 21.7 (the same, and a clear and a fold of 4-byte counters),
+// partitioned 5.4 / 20.0 (two parses more), so the other two run only when
+// asked for.  A fourth way, rebinning every event into a 4-byte record in
+// stream order and adding the records in a separate pass with 30 registers a
+// thread (eight blocks per SM, more adds in flight), was slower as well: the
+// adds are bound by the DRAM sectors they read and write, not by how many are
+// in flight.
 constexpr bool kPartitionedByDefault = false;
 constexpr long long kPartitionMinWords = 1LL << 24;
 constexpr bool kWideByDefault = false;
@@ -103,125 +104,107 @@ __device__ __forceinline__ int ewtype(uint32_t ew1, uint32_t ew2) {
   return (kEwTypes >> (2 * (((ew1 >> 30) << 2) | (ew2 >> 30)))) & 3;
 }
 
-// A thread's parse summary: bit e of `map` = exit offset when entering at e;
-// c0 / c1 = time tags seen when entering at 0 / 1.
-struct Sub {
-  uint32_t map, c0, c1;
-};
-__device__ __forceinline__ Sub compose(const Sub &a, const Sub &b) {  // a then b
-  const uint32_t a0 = a.map & 1, a1 = (a.map >> 1) & 1;
-  Sub h;
-  h.map = ((b.map >> a0) & 1) | (((b.map >> a1) & 1) << 1);
-  h.c0 = a.c0 + (a0 ? b.c1 : b.c0);
-  h.c1 = a.c1 + (a1 ? b.c1 : b.c0);
-  return h;
-}
 __device__ __forceinline__ bool is_timetag(uint32_t ew1, uint32_t ew2) {
   const uint32_t tag = (ew1 & 0xffff) | ((ew2 & 0xffff) << 16);
   return (tag & 0xE0000000u) == 0x80000000u;
 }
 
-// Parse positions [s + e, s + kSub) of the staged tile; `pend` is where the
-// packet (or the stream) ends, relative to the tile.
-__device__ __forceinline__ void sub_parse(const uint32_t *w, int s, int e, int pend, uint32_t &exit_off,
-                                          uint32_t &ntags) {
-  int pos = s + e;
-  ntags = 0;
-  while (pos < s + kSub) {
-    if (pos + 1 >= pend) {  // the packet's last word has no partner
-      exit_off = 0;
-      return;
-    }
-    const uint32_t a = w[pos], b = w[pos + 1];
-    const int t = ewtype(a, b);
-    if (t == 2 && is_timetag(a, b)) ntags++;
-    pos += (t == 3) ? 1 : 2;
-  }
-  exit_off = (uint32_t)(pos - (s + kSub));
+// The words of a thread: run r holds the tile's words rel(r) .. rel(r) + 3,
+// nx[r] the word after them.  A warp owns 512 consecutive words, run by run.
+struct LmRuns {
+  uint4 v[kRuns];
+  uint32_t nx[kRuns];
+};
+__device__ __forceinline__ int run_rel(int r) {
+  return ((int)(threadIdx.x >> 5) * (kRuns * 32) + r * 32 + (int)(threadIdx.x & 31)) * 4;
 }
 
-__device__ __forceinline__ Sub sub_summary(const uint32_t *w, int s, int pend) {
-  Sub r;
-  uint32_t x0, x1;
-  sub_parse(w, s, 0, pend, x0, r.c0);
-  sub_parse(w, s, 1, pend, x1, r.c1);
-  r.map = x0 | (x1 << 1);
-  return r;
-}
-
-__device__ __forceinline__ Sub shfl_up_sub(const Sub &v, int d) {
-  Sub o;
-  o.map = __shfl_up_sync(0xffffffffu, v.map, d);
-  o.c0 = __shfl_up_sync(0xffffffffu, v.c0, d);
-  o.c1 = __shfl_up_sync(0xffffffffu, v.c1, d);
-  return o;
-}
-
-// Inclusive block scan of Sub (composition in thread order); also returns
-// the exclusive prefix of this thread.  Identity: map 0b10 (0->0, 1->1).
-__device__ void block_scan(Sub v, Sub &incl, Sub &excl, Sub *warp_tot) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  Sub x = v;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const Sub o = shfl_up_sub(x, d);
-    if (lane >= d) x = compose(o, x);
-  }
-  if (lane == 31) warp_tot[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    Sub t = lane < kThreads / 32 ? warp_tot[lane] : Sub{2u, 0u, 0u};
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const Sub o = shfl_up_sub(t, d);
-      if (lane >= d) t = compose(o, t);
-    }
-    if (lane < kThreads / 32) warp_tot[lane] = t;  // inclusive over warps
-  }
-  __syncthreads();
-  incl = (wid > 0) ? compose(warp_tot[wid - 1], x) : x;
-  const Sub prev_lane = shfl_up_sub(x, 1);
-  const Sub in_warp = (lane > 0) ? prev_lane : Sub{2u, 0u, 0u};
-  excl = (wid > 0) ? compose(warp_tot[wid - 1], in_warp) : in_warp;
-}
-
-// Stage the tile (plus one halo word) in shared memory; returns `pend`.
-__device__ __forceinline__ int stage_tile(const uint32_t *__restrict__ words, long long n, long long t0, uint32_t *w) {
+// Load the tile at t0; returns where its packet (or the stream) ends relative
+// to t0, at most kTileWords + 2.  Words from there on read as 0.
+__device__ __forceinline__ int load_runs(const uint32_t *__restrict__ words, long long n, long long t0, LmRuns &q) {
   const long long pkt_end = (t0 / kPacketWords + 1) * kPacketWords;
-  const long long lim = pkt_end < n ? pkt_end : n;
-  const long long avail = lim - t0;
-  const int pend = (int)(avail < kTileWords + 1 ? avail : (long long)kTileWords + 1);
-  const uint4 *src = reinterpret_cast<const uint4 *>(words + t0);
-  const int nvec = (pend >= kTileWords) ? kTileWords / 4 : pend / 4;
-  for (int i = threadIdx.x; i < nvec; i += kThreads) reinterpret_cast<uint4 *>(w)[i] = __ldg(src + i);
-  for (int i = nvec * 4 + threadIdx.x; i < pend; i += kThreads) w[i] = __ldg(words + t0 + i);
-  for (int i = pend + threadIdx.x; i < kTileWords + 1; i += kThreads) w[i] = 0u;
-  __syncthreads();
+  const long long avail = (pkt_end < n ? pkt_end : n) - t0;
+  const int pend = (int)(avail < kTileWords + 2 ? avail : (long long)kTileWords + 2);
+  const uint32_t *p = words + t0;
+  const bool last = (threadIdx.x & 31) == 31;
+#pragma unroll
+  for (int r = 0; r < kRuns; r++) {
+    const int rel = run_rel(r);
+    if (rel + 4 <= pend) {
+      q.v[r] = __ldg(reinterpret_cast<const uint4 *>(p + rel));
+    } else {
+      q.v[r].x = rel < pend ? __ldg(p + rel) : 0u;
+      q.v[r].y = rel + 1 < pend ? __ldg(p + rel + 1) : 0u;
+      q.v[r].z = rel + 2 < pend ? __ldg(p + rel + 2) : 0u;
+      q.v[r].w = 0u;
+    }
+    q.nx[r] = last && rel + 4 < pend ? __ldg(p + rel + 4) : 0u;
+  }
+#pragma unroll
+  for (int r = 0; r < kRuns; r++) {
+    const uint32_t o = __shfl_down_sync(0xffffffffu, q.v[r].x, 1);
+    if (!last) q.nx[r] = o;
+  }
   return pend;
 }
 
-__global__ void __launch_bounds__(kThreads) lm_map_kernel(const uint32_t *__restrict__ words, long long n,
-                                                          unsigned long long *__restrict__ tile_sum) {
-  __shared__ __align__(16) uint32_t w[kTileWords + 4];
-  __shared__ Sub wt[32];
-  const long long t0 = (long long)blockIdx.x * kTileWords;
-  const int pend = stage_tile(words, n, t0, w);
-  const Sub v = sub_summary(w, threadIdx.x * kSub, pend);
-  Sub incl, excl;
-  block_scan(v, incl, excl, wt);
-  if (threadIdx.x == kThreads - 1)
-    tile_sum[blockIdx.x] = (unsigned long long)incl.map | ((unsigned long long)incl.c0 << 16) |
-                           ((unsigned long long)incl.c1 << 40);
+// Bit k: an event (a pair that is in sync) starts at word k of run r.
+__device__ __forceinline__ uint32_t run_events(const LmRuns &q, int r, int pend) {
+  const uint4 v = q.v[r];
+  uint32_t m = ((~v.x & v.y) >> 31) | (((~v.y & v.z) >> 31) << 1) | (((~v.z & v.w) >> 31) << 2) |
+               (((~v.w & q.nx[r]) >> 31) << 3);
+  const int left = pend - 1 - run_rel(r);  // words that have a partner
+  if (left < 4) m &= left > 0 ? (1u << left) - 1u : 0u;
+  return m;
 }
 
-// One warp per packet: tile entries and tag offsets within the packet.  Each
-// lane composes the summaries of its run of tiles, a warp scan gives every
-// run its entry (a packet is parsed from its first word: entry 0) and tag
-// offset, and the lane walks its run again to write them.
+// Events never start on adjacent words, so half h of a run (words 2h, 2h + 1)
+// starts one at most; returns its word (0..3), -1 without one.
+__device__ __forceinline__ int run_event(const LmRuns &q, int r, uint32_t m, int h, uint32_t &a, uint32_t &b) {
+  const uint4 v = q.v[r];
+  const uint32_t w0 = h ? v.z : v.x, w1 = h ? v.w : v.y, w2 = h ? q.nx[r] : v.z;
+  const uint32_t at = (m >> (2 * h)) & 3u;
+  a = (at & 2u) ? w1 : w0;
+  b = (at & 2u) ? w2 : w1;
+  return at ? 2 * h + (int)(at >> 1) : -1;
+}
+
+__device__ __forceinline__ uint32_t run_timetags(const LmRuns &q, int r, uint32_t m) {
+  uint32_t n = 0;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    uint32_t a, b;
+    if (run_event(q, r, m, h, a, b) >= 0 && ewtype(a, b) == 2 && is_timetag(a, b)) n++;
+  }
+  return n;
+}
+
+__global__ void __launch_bounds__(kThreads) lm_map_kernel(const uint32_t *__restrict__ words, long long n,
+                                                          unsigned int *__restrict__ tile_tags) {
+  // Bound by the read of the stream: 0.8 GB in 167 us (parsed word by word
+  // from shared memory, from both entries, with a block scan: 784).
+  __shared__ unsigned int wt[kThreads / 32];
+  LmRuns q;
+  const int pend = load_runs(words, n, (long long)blockIdx.x * kTileWords, q);
+  uint32_t c = 0;
+#pragma unroll
+  for (int r = 0; r < kRuns; r++) c += run_timetags(q, r, run_events(q, r, pend));
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) wt[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned int t = 0;
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; i++) t += wt[i];
+    tile_tags[blockIdx.x] = t;
+  }
+}
+
+// One warp per packet: the tag offsets of its tiles within it.
 constexpr int kEntryThreads = 128;
-__global__ void __launch_bounds__(kEntryThreads) lm_entry_kernel(const unsigned long long *__restrict__ tile_sum,
+__global__ void __launch_bounds__(kEntryThreads) lm_entry_kernel(const unsigned int *__restrict__ tile_tags,
                                                                  long long ntiles, int tiles_per_packet,
-                                                                 long long npackets, uint8_t *__restrict__ tile_entry,
+                                                                 long long npackets,
                                                                  unsigned int *__restrict__ tile_tagoff,
                                                                  unsigned long long *__restrict__ packet_tags) {
   const long long p = ((long long)blockIdx.x * kEntryThreads + threadIdx.x) >> 5;  // the same in the whole warp
@@ -229,31 +212,20 @@ __global__ void __launch_bounds__(kEntryThreads) lm_entry_kernel(const unsigned 
   if (p >= npackets) return;
   const long long t_begin = p * tiles_per_packet;
   const long long t_end = min(t_begin + tiles_per_packet, ntiles);
-  const int per = (tiles_per_packet + 31) / 32;
-  const long long lb = min(t_begin + (long long)lane * per, t_end), le = min(lb + per, t_end);
-  auto tile = [](unsigned long long s) {
-    return Sub{(uint32_t)(s & 3u), (uint32_t)((s >> 16) & 0xFFFFFF), (uint32_t)((s >> 40) & 0xFFFFFF)};
-  };
-  Sub run{2u, 0u, 0u};  // identity: 0 -> 0, 1 -> 1
-  for (long long t = lb; t < le; t++) run = compose(run, tile(tile_sum[t]));
-  Sub incl = run;
+  unsigned int run = 0;
+  for (long long tb = t_begin; tb < t_end; tb += 32) {
+    const long long t = tb + lane;
+    const unsigned int c = t < t_end ? tile_tags[t] : 0u;
+    unsigned int incl = c;
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const Sub o = shfl_up_sub(incl, d);
-    if (lane >= d) incl = compose(o, incl);
+    for (int d = 1; d < 32; d <<= 1) {
+      const unsigned int o = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += o;
+    }
+    if (t < t_end) tile_tagoff[t] = run + incl - c;
+    run += __shfl_sync(0xffffffffu, incl, 31);
   }
-  const Sub prev = shfl_up_sub(incl, 1);
-  const Sub excl = lane > 0 ? prev : Sub{2u, 0u, 0u};
-  uint32_t e = excl.map & 1u;  // entering the packet at offset 0
-  unsigned long long off = excl.c0;
-  for (long long t = lb; t < le; t++) {
-    const unsigned long long s = tile_sum[t];
-    tile_entry[t] = (uint8_t)e;
-    tile_tagoff[t] = (unsigned int)off;
-    off += e ? ((s >> 40) & 0xFFFFFF) : ((s >> 16) & 0xFFFFFF);
-    e = (uint32_t)((s >> e) & 1);
-  }
-  if (lane == 31) packet_tags[p] = incl.c0;
+  if (lane == 0) packet_tags[p] = run;
 }
 
 // Exclusive scan of the per-packet tag counts (one block).
@@ -300,8 +272,8 @@ struct LmShared {
 
 // rebin_event (LM_Rebinner_mp.cpp:188-219) in two halves: the LUT entry of a
 // crystal pair, then the address (or -1) from that entry.
-__device__ __forceinline__ size_t sol_index(int mp, int al, int ax, int bl, int bx) {
-  return ((size_t)mp * 144 + ax + 72 * al) * 144 + bx + 72 * bl;
+__device__ __forceinline__ int sol_index(int mp, int al, int ax, int bl, int bx) {
+  return (mp * 144 + ax + 72 * al) * 144 + bx + 72 * bl;
 }
 __device__ __forceinline__ long long rebin_address(const LmDev &g, const LmShared &t, const hrrt::LmSol &s, int ay,
                                                    int by) {
@@ -323,51 +295,63 @@ __device__ __forceinline__ long long rebin_address(const LmDev &g, const LmShare
 constexpr int kPartShift = 25;
 constexpr int kMaxParts = 64;
 
-// Walk one thread's words from its entry offset: count the statistics (kStats),
-// record time tags in stream order (when tags != null), and hand every
-// histogrammed event to emit(address, sinogram 0/1, subtract) -- the
-// coincidence events together, to emit_events(addresses, live, sinogram-1
-// and subtract bit masks).  The parse
-// runs first and notes where the thread's coincidence events start (at most
-// kSub/2 of them); the events are then decoded and rebinned in an unrolled
-// pass whose LUT loads are independent of one another.  Emission order does
-// not matter: the bins are sums modulo 2^16 and the statistics counts.
+// Take one thread's words: count the statistics (kStats), record time tags in
+// stream order (when tags != null), and hand every histogrammed event to
+// emit(address, sinogram 0/1, subtract) -- the coincidence events together, to
+// emit_events(addresses, live, sinogram-1 and subtract bit masks).  Slot 2 r +
+// h is half h of run r (run_event); the slots are decoded and rebinned in
+// unrolled passes whose LUT loads are independent of one another.  `limit` is
+// relative to the tile; the time tags before run r number tagpos0 + pre[r].
+// Emission order does not matter: the bins are sums modulo 2^16 and the
+// statistics counts.
 template <bool kStats, typename Emit, typename EmitEvents>
-__device__ __forceinline__ void walk_events(const LmDev &g, const LmShared &t, const uint32_t *w, int s, int e,
-                                            int pend, long long t0, long long limit, int mode, int flags,
-                                            uint32_t (&c)[kStCount], unsigned long long tagpos, long long tag_cap,
+__device__ __forceinline__ void walk_events(const LmDev &g, const LmShared &t, const LmRuns &q, int pend,
+                                            long long t0, int limit, int mode, int flags,
+                                            uint32_t (&c)[kStCount], unsigned long long tagpos0,
+                                            const uint32_t (&pre)[kRuns], long long tag_cap,
                                             longlong2 *__restrict__ tags, Emit emit, EmitEvents emit_events) {
   const bool doi = (flags & HRRT_LM_NO_DOI) == 0;
   const bool border = (flags & HRRT_LM_IGNORE_BORDER_CRYSTAL) != 0;
   const int xhigh = border ? 71 : 72;
-  uint32_t evmask = 0;  // bit k: an event (below the limit) starts at word s + k
-  uint32_t ttmask = 0;  // bit k: a time tag starts at word s + k (head curve)
-  const unsigned long long tagpos0 = tagpos;
-  int pos = s + e;
-  while (pos < s + kSub) {
-    if (pos + 1 >= pend) break;
-    const long long gp = t0 + pos;
-    const uint32_t ew1 = w[pos], ew2 = w[pos + 1];
-    const int type = ewtype(ew1, ew2);
-    if (type == 3) {
-      if (kStats && gp < limit) c[kStResync]++;
-      pos += 1;
-      continue;
+  uint32_t ttmask = 0;  // bit k: slot k holds a time tag (head curve)
+  // coincidence events (rebin_packet, histogram_mp.cpp:1114-1225): decode,
+  // reject, LUT entry ...
+  int idx[kEv];
+  uint32_t need = 0, delayed = 0;  // bit k: slot k is rebinned / is delayed
+  uint32_t yy[kEv];                // ay | by << 16
+#pragma unroll
+  for (int k = 0; k < kEv; k++) {
+    const int r = k >> 1, h = k & 1;
+    const uint32_t ev = run_events(q, r, pend);
+    if (kStats && h == 0) {
+      // resynchronisations: words with a partner, below the limit, that are
+      // neither an event's first word nor its second
+      const int top = min(limit, pend - 1) - run_rel(r);  // words of the run (and on) that count
+      if (top > 0) {
+        const uint32_t in = top < 4 ? (1u << top) - 1u : 0xFu, in2 = top < 5 ? (1u << (top - 1)) - 1u : 0xFu;
+        c[kStResync] += __popc(in) - __popc(ev & in) - __popc(ev & in2);
+      }
     }
-    pos += 2;
+    idx[k] = 0;
+    yy[k] = 0;
+    uint32_t ew1, ew2;
+    const int at = run_event(q, r, ev, h, ew1, ew2);
+    if (at < 0) continue;
+    const int rel = run_rel(r) + at;
+    const int type = ewtype(ew1, ew2);
     if (type == 2) {
       const uint32_t tag = (ew1 & 0xffff) | ((ew2 & 0xffff) << 16);
       const bool timetag = (tag & 0xE0000000u) == 0x80000000u;
+      const unsigned long long tagpos = tagpos0 + pre[r] + (h ? (ttmask >> (2 * r)) & 1u : 0u);
       if (timetag) {
-        if (tags && (long long)tagpos < tag_cap) tags[tagpos] = make_longlong2(gp, (long long)tag);
-        tagpos++;
-        ttmask |= 1u << (pos - 2 - s);
+        if (tags && (long long)tagpos < tag_cap) tags[tagpos] = make_longlong2(t0 + rel, (long long)tag);
+        ttmask |= 1u << k;
       } else if (tags && g.sing && (tag & 0xE0000000u) == 0xA0000000u) {
         // block singles (process_tagword, histogram_mp.cpp:260-270), in stream order later
-        const unsigned int k = atomicAdd(g.sing_n, 1u);
-        if ((long long)k < g.sing_cap) g.sing[k] = make_longlong2(gp, (long long)tag);
+        const unsigned int i = atomicAdd(g.sing_n, 1u);
+        if ((long long)i < g.sing_cap) g.sing[i] = make_longlong2(t0 + rel, (long long)tag);
       }
-      if (gp >= limit) continue;
+      if (rel >= limit) continue;
       if (kStats) {
         c[kStTags]++;
         if (timetag) c[kStTimetags]++;
@@ -391,26 +375,7 @@ __device__ __forceinline__ void walk_events(const LmDev &g, const LmShared &t, c
       }
       continue;
     }
-    if (gp >= limit) continue;
-    evmask |= 1u << (pos - 2 - s);
-  }
-  if (!evmask) return;
-  // coincidence events (rebin_packet, histogram_mp.cpp:1114-1225): decode,
-  // reject, LUT entry ...
-  constexpr int kEv = kSub / 2;
-  size_t idx[kEv];
-  uint32_t need = 0, delayed = 0;  // bit k: event k is rebinned / is delayed
-  int ays[kEv], bys[kEv];
-  uint32_t m = evmask;
-#pragma unroll
-  for (int k = 0; k < kEv; k++) {
-    idx[k] = 0;
-    ays[k] = bys[k] = 0;
-    if (!m) continue;
-    const int p = __ffs(m) - 1;
-    m &= m - 1;
-    const uint32_t ew1 = w[s + p], ew2 = w[s + p + 1];
-    const int type = ewtype(ew1, ew2);
+    if (rel >= limit) continue;
     const int mpe = ((ew1 >> 16) & 7) | (((ew2 >> 16) & 7) << 3);
     const int ax = ew1 & 0xff, ay = (ew1 >> 8) & 0xff, bx = ew2 & 0xff, by = (ew2 >> 8) & 0xff;
     const int doia = doi ? (int)((ew1 >> 22) & 7) : 1, doib = doi ? (int)((ew2 >> 22) & 7) : 1;
@@ -439,8 +404,7 @@ __device__ __forceinline__ void walk_events(const LmDev &g, const LmShared &t, c
       continue;
     }
     idx[k] = sol_index(mpe, doia, ax, doib, bx);
-    ays[k] = ay;
-    bys[k] = by;
+    yy[k] = (uint32_t)ay | ((uint32_t)by << 16);
     need |= 1u << k;
     if (type != 0) delayed |= 1u << k;
   }
@@ -455,14 +419,11 @@ __device__ __forceinline__ void walk_events(const LmDev &g, const LmShared &t, c
   // head curve: each event counts towards the interval of the time tags
   // before it, accumulated while the interval stays the same
   unsigned long long hc_iv = ~0ull, hc_p = 0, hc_d = 0;
-  uint32_t m2 = evmask;
 #pragma unroll
   for (int k = 0; k < kEv; k++) {
     addr[k] = 0;
-    const int p = m2 ? __ffs(m2) - 1 : 0;
-    if (m2) m2 &= m2 - 1;
     if (!((need >> k) & 1)) continue;
-    const long long a = rebin_address(g, t, sol[k], ays[k], bys[k]);
+    const long long a = rebin_address(g, t, sol[k], (int)(yy[k] & 0xffffu), (int)(yy[k] >> 16));
     if (a < 0) {
       if (kStats) c[kStUnmapped]++;
       continue;
@@ -474,7 +435,7 @@ __device__ __forceinline__ void walk_events(const LmDev &g, const LmShared &t, c
       else
         c[kStPrompts]++;
       if (g.ivl) {
-        const unsigned long long iv = tagpos0 + __popc(ttmask & ((1u << p) - 1u));
+        const unsigned long long iv = tagpos0 + pre[k >> 1] + ((k & 1) ? (ttmask >> (k - 1)) & 1u : 0u);
         if (iv != hc_iv) {
           if (hc_iv != ~0ull) {
             if (hc_p) atomicAdd(g.ivl + 2 * hc_iv, hc_p);
@@ -506,7 +467,6 @@ __device__ __forceinline__ void walk_events(const LmDev &g, const LmShared &t, c
 
 // The direct histogram of a thread's events: every add issued before any
 // carry is checked, so the read-modify-writes are in flight together.
-template <int kEv>
 __device__ __forceinline__ void bump16_events(uint32_t *__restrict__ sino, uint32_t *__restrict__ dly,
                                               const long long (&addr)[kEv], uint32_t live, uint32_t sel,
                                               uint32_t minus) {
@@ -533,6 +493,11 @@ __device__ __forceinline__ void bump16_events(uint32_t *__restrict__ sino, uint3
   }
 }
 
+// Bound by the random read-modify-writes: 100 M events in 4.19 ms, 24 G a
+// second, each fetching 64 bytes of a sinogram from DRAM (the parse from
+// shared memory, whose 16-word stride met 16-way bank conflicts, with a block
+// scan of entry maps: 4.45 ms).
+//
 // kMode 0: time tags only; 1: histogram directly (atomics into the 16-bit
 // bins); 2: count events per histogram partition; 3: scatter packed event
 // records (address | sinogram << 29 | subtract << 30) partition-major; 4:
@@ -540,17 +505,16 @@ __device__ __forceinline__ void bump16_events(uint32_t *__restrict__ sino, uint3
 // carry to check, so no read-modify-write round trip per event), folded into
 // the 16-bit bins afterwards.  Statistics are counted by modes 1, 2 and 4.
 #ifndef HRRT_LM_MIN_BLOCKS
-#define HRRT_LM_MIN_BLOCKS 3  // 4 and 5 (64 and 48 registers, with spills) measured slower on B200
+#define HRRT_LM_MIN_BLOCKS 3  // 2 (84 registers) 4630 us, 3 (74) 4187, 4 (64, with spills) 4177 for 100 M events
 #endif
 template <int kMode>
 __global__ void __launch_bounds__(kThreads, HRRT_LM_MIN_BLOCKS) lm_hist_kernel(
-    LmDev g, const uint32_t *__restrict__ words, long long n, const uint8_t *__restrict__ tile_entry,
+    LmDev g, const uint32_t *__restrict__ words, long long n,
     const unsigned int *__restrict__ tile_tagoff, const unsigned long long *__restrict__ packet_tagoff,
     int tiles_per_packet, long long limit, int mode, int flags, long long tag_cap, longlong2 *__restrict__ tags,
     uint32_t *__restrict__ sino, uint32_t *__restrict__ dly, unsigned long long *__restrict__ stats,
     unsigned long long *__restrict__ part_cursor, uint32_t *__restrict__ records, int parts_per_sino) {
-  __shared__ __align__(16) uint32_t w[kTileWords + 4];
-  __shared__ Sub wt[32];
+  __shared__ unsigned int wt[kThreads / 32];
   __shared__ LmShared tb;
   __shared__ unsigned long long st[kStCount];
   __shared__ unsigned int pcount[kMaxParts];
@@ -568,15 +532,34 @@ __global__ void __launch_bounds__(kThreads, HRRT_LM_MIN_BLOCKS) lm_hist_kernel(
   if (threadIdx.x < kMaxParts) pcount[threadIdx.x] = 0;
   const long long tile = blockIdx.x;
   const long long t0 = tile * kTileWords;
-  const int pend = stage_tile(words, n, t0, w);
-  const int s = threadIdx.x * kSub;
-  const Sub v = sub_summary(w, s, pend);
-  Sub incl, excl;
-  block_scan(v, incl, excl, wt);
-  const uint32_t te = tile_entry[tile];
-  const int e = (int)((excl.map >> te) & 1);
-  const unsigned long long tagpos =
-      packet_tagoff[tile / tiles_per_packet] + tile_tagoff[tile] + (te ? excl.c1 : excl.c0);
+  LmRuns q;
+  const int pend = load_runs(words, n, t0, q);
+  const int lim = (int)max(-1ll, min(limit - t0, (long long)kTileWords + 2));
+  // the time tags before each run, where they are written or count intervals
+  uint32_t pre[kRuns] = {0, 0, 0, 0};
+  unsigned long long tagpos = 0;
+  if (tag_cap > 0 || g.ivl) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t run = 0;
+#pragma unroll
+    for (int r = 0; r < kRuns; r++) {
+      const uint32_t k = run_timetags(q, r, run_events(q, r, pend));
+      const uint32_t b1 = __ballot_sync(0xffffffffu, k > 0), b2 = __ballot_sync(0xffffffffu, k > 1);
+      pre[r] = run + __popc(b1 & below) + __popc(b2 & below);
+      run += __popc(b1) + __popc(b2);
+    }
+    if (lane == 0) wt[wid] = run;
+    __syncthreads();
+    uint32_t before = 0;
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; i++) before += i < wid ? wt[i] : 0u;
+#pragma unroll
+    for (int r = 0; r < kRuns; r++) pre[r] += before;
+    tagpos = packet_tagoff[tile / tiles_per_packet] + tile_tagoff[tile];
+  } else {
+    __syncthreads();
+  }
   longlong2 *tg = tag_cap > 0 ? tags : nullptr;
   uint32_t c[kStCount] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   auto part_of = [&](long long addr, int sel) { return sel * parts_per_sino + (int)(addr >> kPartShift); };
@@ -584,32 +567,32 @@ __global__ void __launch_bounds__(kThreads, HRRT_LM_MIN_BLOCKS) lm_hist_kernel(
   auto each = [](auto f) {
     return [f](const auto &a, uint32_t live, uint32_t sel, uint32_t minus) {
 #pragma unroll
-      for (int k = 0; k < kSub / 2; k++)
+      for (int k = 0; k < kEv; k++)
         if ((live >> k) & 1) f(a[k], (int)((sel >> k) & 1), ((minus >> k) & 1) != 0);
     };
   };
   if (kMode == 0) {
     auto none = [](long long, int, bool) {};
-    walk_events<false>(g, tb, w, s, e, pend, t0, limit, mode, flags, c, tagpos, tag_cap, tg, none, each(none));
+    walk_events<false>(g, tb, q, pend, t0, lim, mode, flags, c, tagpos, pre, tag_cap, tg, none, each(none));
   } else if (kMode == 1) {
-    walk_events<true>(g, tb, w, s, e, pend, t0, limit, mode, flags, c, tagpos, tag_cap, tg,
+    walk_events<true>(g, tb, q, pend, t0, lim, mode, flags, c, tagpos, pre, tag_cap, tg,
                       [&](long long addr, int sel, bool minus) { bump16(sel ? dly : sino, addr, minus); },
-                      [&](const long long (&a)[kSub / 2], uint32_t live, uint32_t sel, uint32_t minus) {
-                        bump16_events<kSub / 2>(sino, dly, a, live, sel, minus);
+                      [&](const long long (&a)[kEv], uint32_t live, uint32_t sel, uint32_t minus) {
+                        bump16_events(sino, dly, a, live, sel, minus);
                       });
   } else if (kMode == 4) {
     int *cs = reinterpret_cast<int *>(records), *cd = cs + g.sino_size;
     auto wide = [&](long long addr, int sel, bool minus) { atomicAdd((sel ? cd : cs) + addr, minus ? -1 : 1); };
-    walk_events<true>(g, tb, w, s, e, pend, t0, limit, mode, flags, c, tagpos, tag_cap, tg, wide, each(wide));
+    walk_events<true>(g, tb, q, pend, t0, lim, mode, flags, c, tagpos, pre, tag_cap, tg, wide, each(wide));
   } else if (kMode == 2) {
     auto count = [&](long long addr, int sel, bool) { atomicAdd(&pcount[part_of(addr, sel)], 1u); };
-    walk_events<true>(g, tb, w, s, e, pend, t0, limit, mode, flags, c, tagpos, tag_cap, tg, count, each(count));
+    walk_events<true>(g, tb, q, pend, t0, lim, mode, flags, c, tagpos, pre, tag_cap, tg, count, each(count));
     __syncthreads();
     if (threadIdx.x < 2 * parts_per_sino && pcount[threadIdx.x])
       atomicAdd(&part_cursor[threadIdx.x], (unsigned long long)pcount[threadIdx.x]);
   } else {
     auto count = [&](long long addr, int sel, bool) { atomicAdd(&pcount[part_of(addr, sel)], 1u); };
-    walk_events<false>(g, tb, w, s, e, pend, t0, limit, mode, flags, c, tagpos, 0, nullptr, count, each(count));
+    walk_events<false>(g, tb, q, pend, t0, lim, mode, flags, c, tagpos, pre, 0, nullptr, count, each(count));
     __syncthreads();
     if (threadIdx.x < 2 * parts_per_sino) {
       const unsigned int k = pcount[threadIdx.x];
@@ -622,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, HRRT_LM_MIN_BLOCKS) lm_hist_kernel(
       const unsigned int k = atomicAdd(&pcount[p], 1u);
       records[pbase[p] + k] = (uint32_t)addr | ((uint32_t)sel << 29) | ((uint32_t)minus << 30);
     };
-    walk_events<false>(g, tb, w, s, e, pend, t0, limit, mode, flags, c, tagpos, 0, nullptr, scatter,
+    walk_events<false>(g, tb, q, pend, t0, lim, mode, flags, c, tagpos, pre, 0, nullptr, scatter,
                        each(scatter));
   }
   if (kMode == 1 || kMode == 2 || kMode == 4) {
@@ -1045,13 +1028,13 @@ int lm_hist_call(hrrt_lm *h, const uint32_t *d_words, long long nwords, int mode
   const long long ntiles = (nwords + kTileWords - 1) / kTileWords;
   const int tpp = (int)(kPacketWords / kTileWords);
   const long long npackets = (nwords + kPacketWords - 1) / kPacketWords;
-  // scratch: tile sums (8), entries (1), tag offsets (4) per tile; packet
-  // offsets (8) per packet; stats.  The time tags get their own buffer once
-  // the scan has counted them.
+  // scratch: tag counts (4) and offsets (4) per tile; packet offsets (8) per
+  // packet; stats.  The time tags get their own buffer once the scan has
+  // counted them.
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  const size_t b_sum = al(8 * ntiles), b_ent = al(ntiles), b_off = al(4 * ntiles), b_pk = al(8 * (npackets + 1)),
+  const size_t b_tag = al(4 * ntiles), b_off = al(4 * ntiles), b_pk = al(8 * (npackets + 1)),
                b_st = al(8 * (kStCount + 1 + 2 * kMaxParts + 1));
-  const size_t need = b_sum + b_ent + b_off + b_pk + b_st;
+  const size_t need = b_tag + b_off + b_pk + b_st;
   if (h->scratch_bytes < need) {
     if (h->scratch) cudaFree(h->scratch);
     h->scratch = nullptr;
@@ -1061,20 +1044,19 @@ int lm_hist_call(hrrt_lm *h, const uint32_t *d_words, long long nwords, int mode
     h->scratch_bytes = need;
   }
   char *p = (char *)h->scratch;
-  auto *tile_sum = (unsigned long long *)p;
-  auto *tile_entry = (uint8_t *)(p + b_sum);
-  auto *tile_tagoff = (unsigned int *)(p + b_sum + b_ent);
-  auto *pk = (unsigned long long *)(p + b_sum + b_ent + b_off);
-  auto *stats = (unsigned long long *)(p + b_sum + b_ent + b_off + b_pk);
+  auto *tile_tags = (unsigned int *)p;
+  auto *tile_tagoff = (unsigned int *)(p + b_tag);
+  auto *pk = (unsigned long long *)(p + b_tag + b_off);
+  auto *stats = (unsigned long long *)(p + b_tag + b_off + b_pk);
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEventCreate(&ev0);
   cudaEventCreate(&ev1);
   cudaEventRecord(ev0, st);
   e = cudaMemsetAsync(stats, 0, 8 * (kStCount + 1), st);
   if (e == cudaSuccess) {
-    lm_map_kernel<<<(unsigned)ntiles, kThreads, 0, st>>>(d_words, nwords, tile_sum);
+    lm_map_kernel<<<(unsigned)ntiles, kThreads, 0, st>>>(d_words, nwords, tile_tags);
     lm_entry_kernel<<<(unsigned)((npackets * 32 + kEntryThreads - 1) / kEntryThreads), kEntryThreads, 0, st>>>(
-        tile_sum, ntiles, tpp, npackets, tile_entry, tile_tagoff, pk);
+        tile_tags, ntiles, tpp, npackets, tile_tagoff, pk);
     lm_scan_kernel<<<1, 1024, 0, st>>>(pk, npackets, stats + kStCount);
     e = cudaGetLastError();
   }
@@ -1142,23 +1124,23 @@ int lm_hist_call(hrrt_lm *h, const uint32_t *d_words, long long nwords, int mode
     uint32_t *sn = (uint32_t *)d_sino, *dl = (uint32_t *)d_delayed;
     switch (kmode) {
       case 0:
-        lm_hist_kernel<0><<<nb, kThreads, 0, st>>>(dv, d_words, nwords, tile_entry, tile_tagoff, pk, tpp, lim,
+        lm_hist_kernel<0><<<nb, kThreads, 0, st>>>(dv, d_words, nwords, tile_tagoff, pk, tpp, lim,
                                                    mode, flags, tcap, tags, sn, dl, stats, cursor, h->records, pps);
         break;
       case 1:
-        lm_hist_kernel<1><<<nb, kThreads, 0, st>>>(dv, d_words, nwords, tile_entry, tile_tagoff, pk, tpp, lim,
+        lm_hist_kernel<1><<<nb, kThreads, 0, st>>>(dv, d_words, nwords, tile_tagoff, pk, tpp, lim,
                                                    mode, flags, tcap, tags, sn, dl, stats, cursor, h->records, pps);
         break;
       case 2:
-        lm_hist_kernel<2><<<nb, kThreads, 0, st>>>(dv, d_words, nwords, tile_entry, tile_tagoff, pk, tpp, lim,
+        lm_hist_kernel<2><<<nb, kThreads, 0, st>>>(dv, d_words, nwords, tile_tagoff, pk, tpp, lim,
                                                    mode, flags, tcap, tags, sn, dl, stats, cursor, h->records, pps);
         break;
       case 4:
-        lm_hist_kernel<4><<<nb, kThreads, 0, st>>>(dv, d_words, nwords, tile_entry, tile_tagoff, pk, tpp, lim,
+        lm_hist_kernel<4><<<nb, kThreads, 0, st>>>(dv, d_words, nwords, tile_tagoff, pk, tpp, lim,
                                                    mode, flags, tcap, tags, sn, dl, stats, cursor, h->records, pps);
         break;
       default:
-        lm_hist_kernel<3><<<nb, kThreads, 0, st>>>(dv, d_words, nwords, tile_entry, tile_tagoff, pk, tpp, lim,
+        lm_hist_kernel<3><<<nb, kThreads, 0, st>>>(dv, d_words, nwords, tile_tagoff, pk, tpp, lim,
                                                    mode, flags, tcap, tags, sn, dl, stats, cursor, h->records, pps);
     }
     return cudaGetLastError();
