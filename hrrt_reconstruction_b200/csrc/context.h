@@ -76,6 +76,7 @@ struct hrrt_ctx {
   int bp_mode = HRRT_BP_REF;
   hrrt::DevGeom dg_adj{};
   int *d_view1 = nullptr;       // one view index, for single-pair entry points
+  hrrt::QuadWork *d_pairwork = nullptr;  // quads of one view pair (projector pair calls)
 
   // a dynamic study using this context's geometry, mult and sensitivity
   struct hrrt_batch *batch = nullptr;

@@ -916,8 +916,11 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
   // projector's own scaling)
   ctx->dg_adj = d;
   ctx->dg_adj.bp_scale = dupload(ctx, std::vector<float>(g.nseg, 1.0f), &e);
+  // the pair calls' view and quads: kept, because an allocation and a free a
+  // call (with its device synchronisation) took longer than the kernels
   ctx->d_view1 = dalloc<int>(ctx, 1, &e);
-  if (!ctx->dg_adj.bp_scale || !ctx->d_view1) return bail(cuda_fail(ctx, e, "adjoint tables"));
+  if (ctx->d_view1) ctx->d_pairwork = dalloc<QuadWork>(ctx, (size_t)g.c + 1, &e);
+  if (!ctx->dg_adj.bp_scale || !ctx->d_pairwork) return bail(cuda_fail(ctx, e, "adjoint tables"));
   int rc = build_work_lists(ctx);
   if (rc) return bail(rc);
   e = cudaStreamSynchronize(ctx->stream);
@@ -1306,8 +1309,9 @@ int hrrt_fp_pair(hrrt_ctx *ctx, const float *image_xyz, int view, float *prj) {
   for (int x = 1; x <= g.c; x++)
     if (g.cyl0[x] != g.cyl1[x] && ctx->nzmask[(size_t)view * nq + x] != 0)
       work.push_back(QuadWork{0, (int16_t)x, (int16_t)view, 0});
-  QuadWork *dw = dupload(ctx, work, &e);
-  if (!dw) return cuda_fail(ctx, e, "work");
+  QuadWork *dw = ctx->d_pairwork;
+  if (!work.empty())
+    CK(cudaMemcpyAsync(dw, work.data(), work.size() * sizeof(QuadWork), cudaMemcpyHostToDevice, ctx->stream), "work");
   CK(cudaMemcpyAsync(ctx->d_tmp_img, image_xyz, ctx->vol * 4, cudaMemcpyHostToDevice, ctx->stream), "fp_pair");
   CK(cudaMemcpyAsync(ctx->d_rows, prj, rows * 4, cudaMemcpyHostToDevice, ctx->stream), "fp_pair");
   {
@@ -1318,8 +1322,6 @@ int hrrt_fp_pair(hrrt_ctx *ctx, const float *image_xyz, int view, float *prj) {
   CK(launch_quad_to_rows(ctx->dg, g.nbins, ctx->d_ratio, dw, (int)work.size(), ctx->d_rows, ctx->stream), "unpack");
   CK(cudaMemcpyAsync(prj, ctx->d_rows, rows * 4, cudaMemcpyDeviceToHost, ctx->stream), "fp_pair");
   CK(cudaStreamSynchronize(ctx->stream), "fp_pair");
-  cudaFree(dw);
-  ctx->allocs.erase(std::find(ctx->allocs.begin(), ctx->allocs.end(), (void *)dw));
   return device_status(ctx);
 }
 int hrrt_forward_project(hrrt_ctx *ctx, const float *image_xyz, float *sino) {
@@ -1519,8 +1521,9 @@ int hrrt_bp_pair(hrrt_ctx *ctx, const float *prj, int view, float *imagebuf_xyz,
   std::vector<QuadWork> work;
   for (int x = 1; x <= g.c; x++)
     if (g.cyl0[x] != g.cyl1[x]) work.push_back(QuadWork{0, (int16_t)x, (int16_t)view, 0});
-  QuadWork *dw = dupload(ctx, work, &e);
-  if (!dw) return cuda_fail(ctx, e, "work");
+  QuadWork *dw = ctx->d_pairwork;
+  if (!work.empty())
+    CK(cudaMemcpyAsync(dw, work.data(), work.size() * sizeof(QuadWork), cudaMemcpyHostToDevice, ctx->stream), "work");
   CK(cudaMemcpyAsync(ctx->d_rows, prj, rows * 4, cudaMemcpyHostToDevice, ctx->stream), "bp_pair");
   CK(cudaMemsetAsync(ctx->d_ratio, 0, ctx->quad_pair * 4, ctx->stream), "bp_pair");
   if (mode == HRRT_BP_ADJOINT) {
@@ -1544,8 +1547,6 @@ int hrrt_bp_pair(hrrt_ctx *ctx, const float *prj, int view, float *imagebuf_xyz,
     }
     CK(cudaMemcpyAsync(imagebuf_xyz, ctx->d_tmp_img, ctx->vol * 4, cudaMemcpyDeviceToHost, ctx->stream), "bp_pair");
     CK(cudaStreamSynchronize(ctx->stream), "bp_pair");
-    cudaFree(dw);
-    ctx->allocs.erase(std::find(ctx->allocs.begin(), ctx->allocs.end(), (void *)dw));
     return device_status(ctx);
   }
   CK(launch_rows_to_quad(ctx->dg, g.nbins, ctx->d_rows, ctx->d_ratio, 1, ctx->stream), "pack");
@@ -1558,8 +1559,6 @@ int hrrt_bp_pair(hrrt_ctx *ctx, const float *prj, int view, float *imagebuf_xyz,
   CK(launch_add_partials(ctx->dg, ctx->d_bc, ctx->d_br, ctx->d_tmp_img, ctx->stream), "add");
   CK(cudaMemcpyAsync(imagebuf_xyz, ctx->d_tmp_img, ctx->vol * 4, cudaMemcpyDeviceToHost, ctx->stream), "bp_pair");
   CK(cudaStreamSynchronize(ctx->stream), "bp_pair");
-  cudaFree(dw);
-  ctx->allocs.erase(std::find(ctx->allocs.begin(), ctx->allocs.end(), (void *)dw));
   return HRRT_OK;
 }
 
@@ -1666,8 +1665,8 @@ int hrrt_rotate_add(hrrt_ctx *ctx, const float *imagebuf_xyz, int view, float *c
   cudaError_t e = cudaSuccess;
   if (!ctx->d_tmp_img) ctx->d_tmp_img = dalloc<float>(ctx, ctx->vol, &e);
   if (!ctx->d_tmp_img) return fail(ctx, HRRT_ERR_NOMEM, "scratch");
-  int *dv = dupload(ctx, std::vector<int>{view}, &e);
-  if (!dv) return cuda_fail(ctx, e, "view");
+  int *dv = ctx->d_view1;
+  CK(cudaMemcpyAsync(dv, &view, sizeof(int), cudaMemcpyHostToDevice, ctx->stream), "view");
   // corr in d_bc[1], imagebuf in d_bc[0]
   CK(cudaMemcpyAsync(ctx->d_bc, imagebuf_xyz, ctx->vol * 4, cudaMemcpyHostToDevice, ctx->stream), "rotate");
   CK(cudaMemcpyAsync(ctx->d_tmp_img, corr_xyz, ctx->vol * 4, cudaMemcpyHostToDevice, ctx->stream), "rotate");
@@ -1678,8 +1677,6 @@ int hrrt_rotate_add(hrrt_ctx *ctx, const float *imagebuf_xyz, int view, float *c
   }
   CK(cudaMemcpyAsync(corr_xyz, ctx->d_tmp_img, ctx->vol * 4, cudaMemcpyDeviceToHost, ctx->stream), "rotate");
   CK(cudaStreamSynchronize(ctx->stream), "rotate");
-  cudaFree(dv);
-  ctx->allocs.erase(std::find(ctx->allocs.begin(), ctx->allocs.end(), (void *)dv));
   return HRRT_OK;
 }
 
