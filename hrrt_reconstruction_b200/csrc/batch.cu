@@ -104,9 +104,9 @@ int time_launch(hrrt_ctx *ctx, int repeats, F fn, double *ms_out) {
   return HRRT_OK;
 }
 
-// Every forward-projection shape (plane variant x producer warps) and
-// back-projection shape of the geometry, timed on subset order[0] with the
-// buffers of `bb`; the fastest of each is kept.
+// Every forward-projection shape (plane variant) of the geometry and the back
+// projector, timed on subset order[0] with the
+// buffers of `bb`; the fastest is kept.
 int autotune(hrrt_ctx *ctx, const SubsetBufs &bb, int repeats, hrrt_tuning *chosen) {
   if (repeats < 1) repeats = 1;
   const int s = ctx->geo.order[0];
@@ -117,28 +117,24 @@ int autotune(hrrt_ctx *ctx, const SubsetBufs &bb, int repeats, hrrt_tuning *chos
   double best_fp = 1e30, best_bp = 1e30;
   for (int vi = 0; vi < 3; vi++) {
     if (!ctx->d_fptasks[vi]) continue;
-    const int cwarps = ctx->fp_offer_warps[vi];
-    for (int pw : {2, 3, 4, 6}) {
-      if (cwarps + pw > kFpVariantWarps[vi]) continue;
-      ProjTune t = saved;
-      t.fp_planes = kFpPlaneVariants[vi];
-      t.fp_pwarps = pw;
-      if (int rc = apply_tune(ctx, t)) return rc;
-      const DevGeom &g = adj ? ctx->dg_adj : ctx->dg;
-      double ms = 0;
-      int rc = time_launch(ctx, repeats, [&] {
-        return launch_fp(g, bb.image, bb.samples, ctx->d_pair_views + (size_t)s * ctx->npairs, 0, ctx->npairs, fw, ctx->fp_cnt[s], 1, bb.prompts, bb.add, ctx->storage, bb.ratio,
-                         ctx->quad_pair, bb.fr, ctx->stream);
-      }, &ms);
-      if (rc) {
-        apply_tune(ctx, saved);
-        return rc;
-      }
-      if (ms < best_fp) {
-        best_fp = ms;
-        best.fp_planes = t.fp_planes;
-        best.fp_pwarps = t.fp_pwarps;
-      }
+    ProjTune t = saved;
+    t.fp_planes = kFpPlaneVariants[vi];
+    t.fp_pwarps = 2;  // every count runs the same kernel; 2 is admitted wherever the variant is
+    if (int rc = apply_tune(ctx, t)) return rc;
+    const DevGeom &g = adj ? ctx->dg_adj : ctx->dg;
+    double ms = 0;
+    int rc = time_launch(ctx, repeats, [&] {
+      return launch_fp(g, bb.image, bb.samples, ctx->d_pair_views + (size_t)s * ctx->npairs, 0, ctx->npairs, fw, ctx->fp_cnt[s], 1, bb.prompts, bb.add, ctx->storage, bb.ratio,
+                       ctx->quad_pair, bb.fr, ctx->stream);
+    }, &ms);
+    if (rc) {
+      apply_tune(ctx, saved);
+      return rc;
+    }
+    if (ms < best_fp) {
+      best_fp = ms;
+      best.fp_planes = t.fp_planes;
+      best.fp_pwarps = t.fp_pwarps;
     }
   }
   if (int rc = apply_tune(ctx, best)) return rc;

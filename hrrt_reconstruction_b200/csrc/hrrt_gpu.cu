@@ -4,9 +4,10 @@
 // inputs (quad layout, every view pair), the image, the per-subset inverse
 // sensitivity images and the per-subset scratch (OP ratio and the two
 // back-projection partials of each view pair of a subset).  One OSEM subset
-// is three launches on the context stream:
-//   fp_kernel (forward projection + ratio) -> bp_kernel -> rotback_kernel
-//   (rotate-back of the nine view pairs fused with the multiplicative update).
+// is four launches on the context stream:
+//   fp_sample_kernel (the rotated rows of the image) -> fp_kernel (forward
+//   projection + ratio) -> bp_kernel -> rotback_kernel (rotate-back of the nine
+//   view pairs fused with the multiplicative update).
 #include <cuda_runtime.h>
 
 #include <algorithm>

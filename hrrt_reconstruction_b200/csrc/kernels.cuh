@@ -156,8 +156,8 @@ inline FrameStrides one_frame() { return FrameStrides{1, nullptr, 0, 0, 0, 0, 0,
 
 // launch shape of the projectors (results do not depend on it)
 struct ProjTune {
-  int fp_planes;  // planes per forward-projection task: 7, 9 or 11 (0: kFpPlanes)
-  int fp_pwarps;  // producer warps of the forward projector (0: as many as fit, 2..6)
+  int fp_planes;  // forward-projection variant: 7, 9 or 11 (0: kFpPlanes), which picks the run (kFpRuns)
+  int fp_pwarps;  // 0 or 2..6: checked and kept, chooses nothing (one warp issues the row copies)
   // the back projector has one shape (a row group of kBpRows rows x kBpZ planes a
   // thread); these are checked and kept, and choose nothing
   int bp_planes;  // 4 or 8 (0: 8)

@@ -267,8 +267,9 @@ int hrrt_reset_kernel_stats(hrrt_ctx *ctx);
 
 /* Results are bit-identical for every shape; only the time changes. */
 typedef struct hrrt_tuning {
-  int fp_planes;          /* planes per forward-projection task: 7, 9 or 11 (0: 9) */
-  int fp_producer_warps;  /* sampling warps of the forward projector: 2..6 (0: as many as fit) */
+  int fp_planes;          /* variant of the forward projector: 7, 9 or 11 (0: 9) -- tasks of 13, 17, 21 or 25 */
+                          /* planes, the larger for the larger number and where segments are many */
+  int fp_producer_warps;  /* 2..6 (0: the library's): checked and kept; the sampling is a kernel of its own */
   int bp_planes;          /* 4 or 8 (0: 8), bp_threads 256 or 384 (0: 384), bp_tile a power of 2 up to 32 (0: */
   int bp_threads;         /* the library's): checked and kept; the back projector has one shape */
   int bp_tile;
