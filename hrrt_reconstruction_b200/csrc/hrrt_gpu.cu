@@ -669,7 +669,7 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
       if (z_lo + d < yb - kBpPad || z_hi + d + 1 > yt + kBpPad) return bail(fail(ctx, HRRT_ERR_ARG, "bp: padding"));
     }
   // the back projector's row groups: per (group, side) the rows kBpRows*m .. +3
-  // (side 1: their mirrors ny - y); rows outside 1..c take the nearest one's
+  // (side 1: their mirrors ny - y); rows outside 1..c-1 take the nearest one's
   // entry and are not stored
   const int bpm = g.c / kBpRows + 1;
   std::vector<BpRows> bprows((size_t)g.groupmax * 2 * bpm);
@@ -678,7 +678,7 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
       for (int m = 0; m < bpm; m++) {
         BpLut l[kBpRows];
         for (int r = 0; r < kBpRows; r++) {
-          const int y = std::min(std::max(kBpRows * m + r, 1), g.c);
+          const int y = std::min(std::max(kBpRows * m + r, 1), g.c - 1);
           l[r] = bpl[(size_t)gg * g.ny + (side ? g.ny - y : y)];
         }
         const size_t at = ((size_t)m * g.groupmax + gg) * 2 + side;
@@ -695,7 +695,7 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
         e.ze = (int16_t)ze;
         e.k = 0;
         for (int r = 0; r < kBpRows; r++) {
-          e.u[r] = l[r].d > lo ? l[r].f : l[r].f - 1.0f;
+          e.f[r] = l[r].f;
           e.k += l[r].d > lo;
         }
         bool wide = hi - lo > 1;

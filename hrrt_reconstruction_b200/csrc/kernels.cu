@@ -552,16 +552,18 @@ __global__ void __launch_bounds__(kFpMaxWarps * 32, 1) fp_kernel(DevGeom g, cons
 // one from the ray of view p+nviews/2 (its row quad); they go to Bc and Br and
 // are added in the rotate-back, which is the reference's assign-then-
 // accumulate order.
-// What bounds it is instruction issue and the latency that 14 warps leave
-// uncovered (FMA pipe about 40 % busy, L1 45 %): per (row group, side of a
+// What bounds it is instruction issue and the latency that 16 warps leave
+// uncovered: per (row group, side of a
 // group) a thread reads 6 shared planes for 16 outputs -- adjacent rows read
 // the segment less than a plane apart, so four rows share a window -- and
-// issues 50 packed FMAs and about 65 other instructions.  One row and 8
+// issues 64 packed FMAs and about as many other instructions.  One row and 8
 // planes a thread (9 shared planes for 8 outputs, an address each) took
-// 1.384 ms a span-3 subset and 0.509 ms a span-9 one; this 0.892 and 0.343.
-// Measured and not used: the row pattern as arithmetic instead of a branch (both
-// slopes applied, one of them 0: 1.021 ms), lane pairs split over two threads
-// for twice the warps (0.941 ms), no prefetch of the next entry (0.977 ms).
+// 1.384 ms a span-3 subset and 0.509 ms a span-9 one; this 0.996 and 0.381,
+// to the same bits.  Measured and not used: one plane for all rows and
+// differences (bp_rows: 0.892 and 0.343 ms; loses sparse data's accuracy), and
+// in that form the row pattern as arithmetic instead of a branch (1.021 ms),
+// lane pairs split over two threads for twice the warps (0.941 ms), no prefetch
+// of the next entry (0.977 ms).
 // ============================================================================
 // The shared planes are stored by phase, plane i at slot bp_slot(i): eight
 // lanes of a warp take consecutive 4-plane runs of one row group, so that
@@ -596,25 +598,26 @@ __device__ __forceinline__ void bp_lerp(Q2 (&s)[KB], const float4 *__restrict__ 
 // one side of a segment group for a row group and a run of planes (BpRows):
 // the first (SIDE 0) or last (SIDE 1) K rows are one plane further on; A[k]
 // is where plane k of the window lies, A[0] + 16 and A[1] + 16 the next two.
-// The differences are fused multiply-adds by a run-time (-1, -1): a packed
-// subtraction costs two more instructions for the signs.
+// Each output adds its lower, then its upper plane by their own weights, as
+// bp_lerp does.  Adding one plane to all rows and the planes' differences to
+// each takes fewer operations (50 packed ones for 64), but cancels where a row
+// gives a large plane next to no weight.
 template <int SIDE, int K>
-__device__ __forceinline__ void bp_rows(Q2 (&s)[kBpRows][kBpZ], Q2 (&com)[kBpZ], const float4 *__restrict__ P,
-                                        const int (&A)[4], const float4 &v, uint64_t neg1) {
-  const uint64_t u[kBpRows] = {pk(v.x, v.x), pk(v.y, v.y), pk(v.z, v.z), pk(v.w, v.w)};
-  Q2 w1 = ldb(P, A[1]), d0 = qfma(ldb(P, A[0]), neg1, w1);
+__device__ __forceinline__ void bp_rows(Q2 (&s)[kBpRows][kBpZ], const float4 *__restrict__ P, const int (&A)[4],
+                                        const float4 &v) {
+  const uint64_t f[kBpRows] = {pk(v.x, v.x), pk(v.y, v.y), pk(v.z, v.z), pk(v.w, v.w)};
+  const uint64_t g[kBpRows] = {pk(1.0f - v.x, 1.0f - v.x), pk(1.0f - v.y, 1.0f - v.y), pk(1.0f - v.z, 1.0f - v.z),
+                               pk(1.0f - v.w, 1.0f - v.w)};
 #pragma unroll
-  for (int j = 0; j < kBpZ; j++) {
-    com[j] = qadd(com[j], w1);
-    Q2 d1 = d0;
-    if (K > 0 || j + 1 < kBpZ) {
-      const Q2 w2 = ldb(P, j == 0 ? A[2] : j == 1 ? A[3] : j == 2 ? A[0] + 16 : A[1] + 16);
-      d1 = qfma(w1, neg1, w2);
-      w1 = w2;
+  for (int k = 0; k < kBpZ + (K > 0 ? 2 : 1); k++) {
+    const Q2 w = ldb(P, k < 4 ? A[k] : A[k - 4] + 16);
+#pragma unroll
+    for (int r = 0; r < kBpRows; r++) {
+      const int on = (SIDE ? r >= kBpRows - K : r < K) ? 1 : 0;
+      const int jl = k - on, ju = jl - 1;
+      if (ju >= 0 && ju < kBpZ) s[r][ju] = qfma(w, f[r], s[r][ju]);
+      if (jl >= 0 && jl < kBpZ) s[r][jl] = qfma(w, g[r], s[r][jl]);
     }
-#pragma unroll
-    for (int r = 0; r < kBpRows; r++) s[r][j] = qfma((SIDE ? r >= kBpRows - K : r < K) ? d1 : d0, u[r], s[r][j]);
-    d0 = d1;
   }
 }
 
@@ -661,20 +664,18 @@ __device__ __forceinline__ void put(float *__restrict__ dst, const Q2 (&s)[kBpZ]
   }
 }
 
-// Two CTAs per SM (their shared planes fill it at span 3) of at most 128
-// registers a thread.  Measured on B200 (span 3 / span 9 subset): 192 threads
-// of 160 registers 941 / 368 us, 224 threads 892 / 361 us, 256 threads
-// 952 / 381 us; one view pair with ACC: 152, 169 and 142 us.
-template <bool ACC>
-constexpr int kBpThreads = ACC ? 256 : 224;
+// Two CTAs per SM (their shared planes fill it at span 3) of 128 registers a
+// thread.  Measured on B200 (span 3 / span 9 subset): 192 threads 1146 / 438
+// us, 224 threads 1005 / 382 us, 256 threads 996 / 381 us.
+constexpr int kBpThreads = 256;
 
 template <bool ACC, bool MULTI>
-__global__ void __launch_bounds__(kBpThreads<ACC>, 2) bp_kernel(DevGeom g, const float4 *__restrict__ in,
+__global__ void __launch_bounds__(kBpThreads, 2) bp_kernel(DevGeom g, const float4 *__restrict__ in,
                                                            long long in_pair_stride, const QuadWork *__restrict__ work,
                                                            float *__restrict__ bc, float *__restrict__ br,
                                                            long long vol, FrameStrides fr, int view0, int x0,
                                                            int split) {
-  constexpr int KB = kBpZ, KR = kBpRows, NT = kBpThreads<ACC>;
+  constexpr int KB = kBpZ, KR = kBpRows, NT = kBpThreads;
   extern __shared__ float4 P[];  // [bp_splanes]: segments with kBpPad zero planes each side
   __shared__ int2 s_base[kFpMaxGroups];  // per group: byte offset of yr 0 of its even / odd segment (of its slot)
   // ACC: one view pair, quads x0.., both partial sums added into bc (each
@@ -711,58 +712,87 @@ __global__ void __launch_bounds__(kBpThreads<ACC>, 2) bp_kernel(DevGeom g, const
   float *bcp = bc + (size_t)w.slot * vol;
   float *brp = (ACC ? bc : br) + (size_t)w.slot * vol;
   const bool vec = ACC && (reinterpret_cast<uintptr_t>(bc) & 15) == 0;
-  const uint64_t neg1 = pk(-g.unit, -g.unit);
   const int ystart = g.cyl0[x], o0 = g.bp_soff[0];
-  const int m0 = ystart / KR, M = c / KR + 1, nm = M - m0, nzc = zp / KB;
+  const int m0 = ystart / KR, nm = max(0, (c - 1) / KR + 1 - m0), nzc = zp / KB;
   // A warp takes 16 consecutive plane runs of one row group in both halves:
-  // half 0 builds sumt1, half 1 sumt2 (the centre row, y = c, has a single
-  // voxel set: half 0's).  The halves read the two segments of a group at the
-  // same position, so a warp's lanes take the same path through bp_rows.
+  // half 0 builds sumt1, half 1 sumt2.  The halves read the two segments of a
+  // group at the same position, so a warp's lanes take the same path through
+  // bp_rows.  The last tiles are 32 plane runs of the centre row, y = c.
   const int lane = threadIdx.x & 31, half = lane >> 4;
   const int CT = (nzc + 15) / 16, tiles = nm * CT;
   const int step = split * (NT / 32);
-  for (int tile = part * (NT / 32) + (threadIdx.x >> 5); tile < tiles; tile += step) {
+  // column voxels (x, yc), (N-x, yc); row voxels (yr, x), (yr, N-x)
+  auto put4 = [&](const Q2 (&v)[KB], int yc, int yr, int z0) {
+    put<ACC>(bcp + ((size_t)x * N + yc) * zp + z0, v, 0, vec);
+    put<ACC>(brp + ((size_t)yr * N + x) * zp + z0, v, 2, vec);
+    if (x != c) {
+      put<ACC>(bcp + ((size_t)(N - x) * N + yc) * zp + z0, v, 1, vec);
+      put<ACC>(brp + ((size_t)yr * N + N - x) * zp + z0, v, 3, vec);
+    }
+  };
+  for (int tile = part * (NT / 32) + (threadIdx.x >> 5); tile < tiles + (nzc + 31) / 32; tile += step) {
+    if (tile >= tiles) {
+      // centre row (sbrt:4260-4284): a single voxel set, rays pass plane
+      // yr = z exactly
+      const int zc = (tile - tiles) * 32 + lane, z0 = zc * KB;
+      if (zc >= nzc) continue;
+      Q2 t[KB];
+#pragma unroll
+      for (int j = 0; j < KB; j++) t[j] = masked ? Q2{0ull, 0ull} : ldq(P + o0 / 4 + zc + j * s4);
+      for (int gg = 0; gg < (masked ? 0 : G); gg++) {
+        const int2 base = s_base[gg];
+        const int yb = g.ybot[2 * gg + 2], yt = g.ytop[2 * gg + 2];
+#pragma unroll
+        for (int j = 0; j < KB; j++) {
+          const int at = 16 * (zc + j * s4);
+          if (z0 + j >= yb && z0 + j <= yt) t[j] = qadd(t[j], qadd(ldb(P, base.x + at), ldb(P, base.y + at)));
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < KB; j++)
+        if (z0 + j >= g.nz) t[j] = Q2{0ull, 0ull};
+      put4(t, c, c, z0);
+      continue;
+    }
     const int ty = tile / CT, tc = tile - ty * CT;
     const int m = m0 + ty, zc = tc * 16 + (lane & 15), z0 = zc * KB;
     if (zc >= nzc) continue;
-    Q2 s[KR][KB], com[KB];
+    Q2 s[KR][KB];
+    // masked quads contribute zero (sbrt:4223-4258, :4595-4640)
 #pragma unroll
     for (int j = 0; j < KB; j++) {
-      com[j] = Q2{0ull, 0ull};
+      s[0][j] = masked ? Q2{0ull, 0ull} : ldq(P + o0 / 4 + zc + j * s4);
 #pragma unroll
-      for (int r = 0; r < KR; r++) s[r][j] = Q2{0ull, 0ull};
+      for (int r = 1; r < KR; r++) s[r][j] = s[0][j];
     }
-    // masked quads contribute zero (sbrt:4223-4258, :4595-4640)
     if (!masked) {
-#pragma unroll
-      for (int j = 0; j < KB; j++) com[j] = ldq(P + o0 / 4 + zc + j * s4);
       const int4 *e = reinterpret_cast<const int4 *>(g.bprows + (size_t)m * G * 2);
       int4 hn = __ldg(e);
-      float4 un = __ldg(reinterpret_cast<const float4 *>(e + 1));
+      float4 fn = __ldg(reinterpret_cast<const float4 *>(e + 1));
       // one side of group gg; sumt1: segment 2k at +u (side 0, rows y) and
       // 2k-1 at -u (side 1, rows N-y); sumt2: the converse
       auto side_of = [&](auto side_c, int gg, int seg, bool last) {
         constexpr int SIDE = decltype(side_c)::value;
         const int4 h = hn;
-        const float4 v = un;
+        const float4 v = fn;
         if (!last) {  // the next entry, in flight under this one's planes
           e += 2;
           hn = __ldg(e);
-          un = __ldg(reinterpret_cast<const float4 *>(e + 1));
+          fn = __ldg(reinterpret_cast<const float4 *>(e + 1));
         }
         if (z0 + KB - 1 < (int)(int16_t)(h.z & 0xffff) || z0 > (h.z >> 16)) return;
         const int B = seg + 16 * zc;
         const int A[4] = {B + 16 * (int)(int16_t)(h.x & 0xffff), B + 16 * (h.x >> 16),
                           B + 16 * (int)(int16_t)(h.y & 0xffff), B + 16 * (h.y >> 16)};
         switch (h.w) {
-          case 0: bp_rows<SIDE, 0>(s, com, P, A, v, neg1); break;
-          case 1: bp_rows<SIDE, 1>(s, com, P, A, v, neg1); break;
-          case 2: bp_rows<SIDE, 2>(s, com, P, A, v, neg1); break;
-          case 3: bp_rows<SIDE, 3>(s, com, P, A, v, neg1); break;
+          case 0: bp_rows<SIDE, 0>(s, P, A, v); break;
+          case 1: bp_rows<SIDE, 1>(s, P, A, v); break;
+          case 2: bp_rows<SIDE, 2>(s, P, A, v); break;
+          case 3: bp_rows<SIDE, 3>(s, P, A, v); break;
           default:
 #pragma unroll
             for (int r = 0; r < KR; r++) {
-              const int y = min(max(KR * m + r, 1), c);
+              const int y = min(max(KR * m + r, 1), c - 1);
               bp_lerp<KB>(s[r], P, s4, seg / 4, g.bplut[(size_t)gg * N + (SIDE ? N - y : y)], z0);
             }
         }
@@ -776,21 +806,12 @@ __global__ void __launch_bounds__(kBpThreads<ACC>, 2) bp_kernel(DevGeom g, const
 #pragma unroll
     for (int r = 0; r < KR; r++) {
       const int y = KR * m + r;
-      if (y < ystart || y > c || (half && y == c)) continue;
+      if (y < ystart || y >= c) continue;
+      // the reference writes planes z < nz only
 #pragma unroll
-      for (int j = 0; j < KB; j++) {
-        // the reference writes planes z < nz only
-        s[r][j] = qadd(s[r][j], com[j]);
+      for (int j = 0; j < KB; j++)
         if (z0 + j >= g.nz) s[r][j] = Q2{0ull, 0ull};
-      }
-      // column voxels (x, yc), (N-x, yc); row voxels (yr, x), (yr, N-x)
-      const int yc = half ? N - y : y, yr = half ? y : N - y;
-      put<ACC>(bcp + ((size_t)x * N + yc) * zp + z0, s[r], 0, vec);
-      put<ACC>(brp + ((size_t)yr * N + x) * zp + z0, s[r], 2, vec);
-      if (x != c) {
-        put<ACC>(bcp + ((size_t)(N - x) * N + yc) * zp + z0, s[r], 1, vec);
-        put<ACC>(brp + ((size_t)yr * N + N - x) * zp + z0, s[r], 3, vec);
-      }
+      put4(s[r], half ? N - y : y, half ? y : N - y, z0);
     }
   }
 }
@@ -1532,7 +1553,7 @@ cudaError_t launch_bp_t(const DevGeom &g, const float *in, long long in_pair_str
   // launches that do not fill the chip share each quad among several CTAs
   const long long quads = (long long)nquads * fr.n;
   const int split = (int)std::max<long long>(1, std::min<long long>(4, (4 * 148 + quads - 1) / quads));
-  k<<<(unsigned)(quads * split), kBpThreads<ACC>, smem, st>>>(g, reinterpret_cast<const float4 *>(in), in_pair_stride / 4,
+  k<<<(unsigned)(quads * split), kBpThreads, smem, st>>>(g, reinterpret_cast<const float4 *>(in), in_pair_stride / 4,
                                                          work, bc, br, vol, fr, view, x0, split);
   return cudaGetLastError();
 }

@@ -71,15 +71,15 @@ struct AdjEnd {
 // One side of a segment group in the back projection of a row group: the rows
 // read the segment at yr = z + shift with a fraction f (BpLut), and the shifts
 // of adjacent rows differ by less than one plane, so that the four rows share
-// a window that starts at the smallest shift d.  With W[k] = p[z + d + k] and
-// D[k] = W[k+1] - W[k], a row whose shift is d + 1 takes W[1] + f*D[1], one
-// whose shift is d takes W[1] + (f-1)*D[0].  Along the rows the shift falls on
-// side 0 and rises on side 1, so the rows at d + 1 are the first or the last k.
+// a window that starts at the smallest shift d.  With W[k] = p[z + d + k], a
+// row whose shift is d + 1 takes (1-f)*W[1] + f*W[2], one whose shift is d
+// takes (1-f)*W[0] + f*W[1].  Along the rows the shift falls on side 0 and
+// rises on side 1, so the rows at d + 1 are the first or the last k.
 struct __align__(16) BpRows {
   int16_t off[4];  // shared slot of plane d + k, from that of plane 0 (bp_slot)
   int16_t zs, ze;  // planes any of the rows takes anything from
   int32_t k;       // rows at d + 1 (0..3), or kBpWide: evaluated row by row
-  float u[4];      // f or f - 1
+  float f[4];
 };
 
 constexpr int kBpWide = 4;
