@@ -1468,19 +1468,33 @@ __global__ void scale_pairs_kernel(DevGeom g, const T *__restrict__ src, const i
   dst[(size_t)slot * dst_pair_stride + i] = o;
 }
 
-// Dynamic shared memory of a kernel that has `ctas` CTAs resident per SM by its
-// registers; what they leave of the SM's memory stays L1, which holds the
-// sampling tables the projectors read (the whole SM's memory as shared memory
-// instead: adjoint 1200 us a subset at span 9 against 1057, back projector 361
-// against 343).
-template <typename K>
-cudaError_t set_smem(K k, size_t smem, int ctas) {
-  constexpr size_t kSm = 228 * 1024, kReserved = 1024;  // of an SM; of a CTA
+// Launches a kernel that has `ctas` CTAs resident per SM by its registers; what
+// their shared memory leaves of the SM's stays L1, which holds the sampling
+// tables the projectors read (the whole SM's memory as shared memory instead:
+// adjoint 1200 us a subset at span 9 against 1057, back projector 361 against
+// 343).  The split goes with the launch, and the limit that belongs to the
+// kernel itself is always the same: contexts of other sizes may launch it from
+// other threads.
+template <typename... P, typename... A>
+cudaError_t launch_smem(void (*k)(P...), long long grid, int threads, size_t smem, int ctas, cudaStream_t st,
+                        A... args) {
+  constexpr size_t kSm = 228 * 1024, kReserved = 1024;        // of an SM; of a CTA
+  constexpr size_t kMaxDynamic = kSm - kReserved - 512;       // less the kernels' static shared memory
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)std::max(smem, kMaxDynamic));
+  if (e != cudaSuccess) return e;
   ctas = (int)std::max<size_t>(1, std::min<size_t>(ctas, kSm / (smem + kReserved)));
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const int pct = (int)std::min<size_t>(100, (ctas * (smem + kReserved) * 100 + kSm - 1) / kSm);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
-  return e;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  at.val.sharedMemCarveout = (unsigned)std::min<size_t>(100, (ctas * (smem + kReserved) * 100 + kSm - 1) / kSm);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
 template <int MODE, int PL, typename PT, typename AT>
@@ -1490,13 +1504,9 @@ cudaError_t launch_fp_t(const DevGeom &g, const float *samples, const QuadWork *
   const int warps = g.nfptasks / 16 + 1;
   const int ZS = g.zp + kFpZPad;
   const size_t smem = (size_t)(2 * kFpSlots + 1) * ZS * sizeof(float4) + (size_t)kFpSlots * g.groupmax * sizeof(FpMid);
-  auto k = fp_kernel<MODE, PL, PT, AT>;
-  cudaError_t e = set_smem(k, smem, std::max(1, 32 / warps));
-  if (e != cudaSuccess) return e;
-  k<<<(unsigned)nwork * fr.n, warps * 32, smem, st>>>(g, reinterpret_cast<const float4 *>(samples), work,
-                                                      (const PT *)prompts, (const AT *)add,
-                                                      reinterpret_cast<float4 *>(out), out_pair_stride / 4, fr);
-  return cudaGetLastError();
+  return launch_smem(fp_kernel<MODE, PL, PT, AT>, (long long)nwork * fr.n, warps * 32, smem, std::max(1, 32 / warps),
+                     st, g, reinterpret_cast<const float4 *>(samples), work, (const PT *)prompts, (const AT *)add,
+                     reinterpret_cast<float4 *>(out), out_pair_stride / 4, fr);
 }
 
 template <int PL>
@@ -1547,15 +1557,11 @@ cudaError_t launch_bp_t(const DevGeom &g, const float *in, long long in_pair_str
                         float *bc, float *br, long long vol, const FrameStrides &fr, int view, int x0,
                         cudaStream_t st) {
   const size_t smem = (size_t)4 * g.bp_s4 * sizeof(float4);
-  auto k = bp_kernel<ACC, MULTI>;
-  cudaError_t e = set_smem(k, smem, 2);
-  if (e != cudaSuccess) return e;
   // launches that do not fill the chip share each quad among several CTAs
   const long long quads = (long long)nquads * fr.n;
   const int split = (int)std::max<long long>(1, std::min<long long>(4, (4 * 148 + quads - 1) / quads));
-  k<<<(unsigned)(quads * split), kBpThreads, smem, st>>>(g, reinterpret_cast<const float4 *>(in), in_pair_stride / 4,
-                                                         work, bc, br, vol, fr, view, x0, split);
-  return cudaGetLastError();
+  return launch_smem(bp_kernel<ACC, MULTI>, quads * split, kBpThreads, smem, 2, st, g,
+                     reinterpret_cast<const float4 *>(in), in_pair_stride / 4, work, bc, br, vol, fr, view, x0, split);
 }
 
 cudaError_t launch_bp(const DevGeom &g, const float *in, long long in_pair_stride, const QuadWork *work, int nwork,
@@ -1570,11 +1576,8 @@ cudaError_t launch_adj(const DevGeom &g, const float *in, long long in_pair_stri
   if (nwork <= 0 || fr.n <= 0) return cudaSuccess;
   const size_t smem = (size_t)g.bp_splanes * sizeof(float4);
   auto k = g.adj_ends ? adj_kernel<kAdjZ, true> : adj_kernel<kAdjZ, false>;
-  cudaError_t e = set_smem(k, smem, 3);
-  if (e != cudaSuccess) return e;
-  k<<<(unsigned)nwork * fr.n, 256, smem, st>>>(g, reinterpret_cast<const float4 *>(in), in_pair_stride / 4, work, bc,
-                                               br, vol, fr);
-  return cudaGetLastError();
+  return launch_smem(k, (long long)nwork * fr.n, 256, smem, 3, st, g, reinterpret_cast<const float4 *>(in),
+                     in_pair_stride / 4, work, bc, br, vol, fr);
 }
 
 cudaError_t launch_adj_rotate(const DevGeom &g, const int *pair_views, int npairs, const float *bc, const float *br,
