@@ -33,7 +33,8 @@ struct hrrt_batch {
   float *images = nullptr;                      // [frame][vol]
   double *sums = nullptr;                       // [frame]
   int group = 1;                                // frames per launch
-  float *ratio = nullptr, *bc = nullptr, *br = nullptr, *samples = nullptr;  // scratch of one group
+  float *ratio = nullptr, *bc = nullptr, *br = nullptr;  // scratch of one group; bc and br [frame][2][npairs][vol]
+  float *samples = nullptr;                     // [frame][npairs][samp_pair][4], or bc where memory is short
   double *partial = nullptr;                    // [group][pb]
   int pb = 0;
   int *d_order = nullptr;                       // [nframes] frames by descending iteration count
@@ -53,19 +54,23 @@ struct hrrt_batch {
   T *alloc(size_t n, cudaError_t *e) {
     void *p = nullptr;
     *e = cudaMalloc(&p, n * sizeof(T) + 16);
-    if (*e != cudaSuccess) return nullptr;
+    if (*e != cudaSuccess) {
+      cudaGetLastError();  // nothing left for the next launch's check
+      return nullptr;
+    }
     allocs.push_back(p);
     return (T *)p;
   }
   FrameStrides strides(int start, int n) const {
+    const long long partials = 2 * (long long)ctx->npairs * ctx->vol;
     return FrameStrides{n,
                         d_order + start,
                         ctx->vol,
                         (long long)in_elems,
                         (long long)ctx->npairs * ctx->quad_pair,
-                        (long long)ctx->npairs * ctx->vol,
+                        partials,
                         (long long)pb,
-                        (long long)ctx->npairs * ctx->dg.samp_pair * 4};
+                        samples == bc ? partials : (long long)ctx->npairs * ctx->dg.samp_pair * 4};
   }
   SubsetBufs bufs(int start, int n) const {
     return SubsetBufs{images, q_prompts, q_add, ratio, bc, br, samples, strides(start, n)};
@@ -138,6 +143,7 @@ int autotune(hrrt_ctx *ctx, const SubsetBufs &bb, int repeats, hrrt_tuning *chos
     }
   }
   if (int rc = apply_tune(ctx, best)) return rc;
+  CK(clear_shared(ctx, bb.samples, bb.bc, ctx->npairs, bb.fr.n), "tune");
   if (!adj) {
     // the back projector has one shape
     int rc = time_launch(ctx, repeats, [&] {
@@ -299,6 +305,7 @@ int hrrt_batch_create(hrrt_ctx *ctx, int nframes, int storage, const float *norm
     return rc;
   };
   cudaError_t e = cudaSuccess;
+  release_samples(ctx);  // the frames have their own
   const size_t flat = (size_t)g.segmentsize * g.nviews * g.nbins;
   for (int i = 0; i < 2; i++) {
     const float *src = i ? atten : norm;
@@ -327,11 +334,12 @@ int hrrt_batch_create(hrrt_ctx *ctx, int nframes, int storage, const float *norm
   const long long fit = free_b > reserve ? (long long)((free_b - reserve) / per) : 0;
   b->group = (int)std::max<long long>(1, std::min<long long>(nframes, fit));
   b->ratio = b->alloc<float>((size_t)b->group * ctx->npairs * ctx->quad_pair, &e);
-  b->bc = b->ratio ? b->alloc<float>((size_t)b->group * ctx->npairs * ctx->vol, &e) : nullptr;
-  b->br = b->bc ? b->alloc<float>((size_t)b->group * ctx->npairs * ctx->vol, &e) : nullptr;
-  b->samples = b->br ? b->alloc<float>((size_t)b->group * samp, &e) : nullptr;
-  b->partial = b->samples ? b->alloc<double>((size_t)b->group * b->pb, &e) : nullptr;
+  b->bc = b->ratio ? b->alloc<float>((size_t)b->group * 2 * ctx->npairs * ctx->vol, &e) : nullptr;
+  if (b->bc) b->br = b->bc + (size_t)ctx->npairs * ctx->vol;
+  b->partial = b->br ? b->alloc<double>((size_t)b->group * b->pb, &e) : nullptr;
   if (!b->partial) return bail(fail(ctx, HRRT_ERR_NOMEM, "batch: scratch"));
+  b->samples = b->alloc<float>((size_t)b->group * samp, &e);
+  if (!b->samples) b->samples = b->bc;
   ctx->batch = b;
   ctx->have_inputs = false;  // the context's single-frame inputs are replaced
   ctx->have_sens = false;

@@ -36,8 +36,13 @@ struct hrrt_ctx {
 
   float *d_image = nullptr;
   float *d_nfinv = nullptr;
-  float *d_ratio = nullptr, *d_bc = nullptr, *d_br = nullptr;
-  float *d_samples = nullptr;   // the forward projector's rotated rows, [npairs][samp_pair][4]
+  float *d_ratio = nullptr;
+  float *d_bc = nullptr, *d_br = nullptr;  // one allocation, [2][npairs][vol]
+  // the forward projector's rotated rows, [npairs][samp_pair][4]: a buffer of
+  // their own once there are inputs; before that, and where memory is short
+  // (samples_shared), the partials' memory, cleared after each projection
+  float *d_samples = nullptr;
+  bool samples_shared = false;
   float *d_tmp_img = nullptr;  // test entry points
   float *d_rows = nullptr;
   double *d_partial = nullptr, *d_sum = nullptr;
@@ -144,10 +149,32 @@ inline int cuda_fail(hrrt_ctx *ctx, cudaError_t e, const char *where) {
     if (e_ != cudaSuccess) return cuda_fail(ctx, e_, where); \
   } while (0)
 
+// gives the rotated rows' own buffer back; false if there is none
+inline bool release_samples(hrrt_ctx *ctx) {
+  if (!ctx->d_samples) return false;
+  cudaFree(ctx->d_samples);
+  ctx->allocs.erase(std::find(ctx->allocs.begin(), ctx->allocs.end(), (void *)ctx->d_samples));
+  ctx->d_samples = nullptr;
+  return true;
+}
+// cudaMalloc that takes that buffer where memory is short, and leaves no
+// error behind for the next launch's check
+inline cudaError_t dmalloc(hrrt_ctx *ctx, void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaSuccess) return e;
+  cudaGetLastError();
+  if (e == cudaErrorMemoryAllocation && release_samples(ctx)) {
+    e = cudaMalloc(p, bytes);
+    ctx->samples_shared = e == cudaSuccess;
+    if (e != cudaSuccess) cudaGetLastError();
+  }
+  return e;
+}
+
 template <typename T>
 inline T *dalloc(hrrt_ctx *ctx, size_t n, cudaError_t *e) {
   void *p = nullptr;
-  *e = cudaMalloc(&p, n * sizeof(T) + 16);
+  *e = dmalloc(ctx, &p, n * sizeof(T) + 16);
   if (*e != cudaSuccess) return nullptr;
   *e = cudaMemsetAsync(p, 0, n * sizeof(T) + 16, ctx->stream);
   ctx->allocs.push_back(p);
@@ -205,6 +232,11 @@ struct SubsetBufs {
 };
 
 // defined in hrrt_gpu.cu
+// where a subset's rotated rows go: their own buffer, the partials without memory for one
+float *samples_of(hrrt_ctx *ctx);
+// the partials are zero beside the field of view's columns: cleared after a
+// projection of `pairs` pairs whose rotated rows lay there (in `frames` blocks)
+cudaError_t clear_shared(const hrrt_ctx *ctx, const float *samples, float *bc, int pairs, int frames);
 SubsetBufs ctx_bufs(hrrt_ctx *ctx);
 // fp -> bp (or the adjoint) -> rotate-back + update of subset s, on ctx->stream
 int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b);

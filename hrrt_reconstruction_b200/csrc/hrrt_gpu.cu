@@ -219,8 +219,26 @@ int build_work_lists(hrrt_ctx *ctx) {
   return HRRT_OK;
 }
 
+float *samples_of(hrrt_ctx *ctx) {
+  if (!ctx->d_samples && !ctx->samples_shared) {
+    cudaError_t e = cudaSuccess;
+    ctx->d_samples = dalloc<float>(ctx, (size_t)ctx->npairs * ctx->dg.samp_pair * 4, &e);
+    ctx->samples_shared = !ctx->d_samples;
+  }
+  return ctx->samples_shared ? ctx->d_bc : ctx->d_samples;
+}
+
+// A pair's rotated rows fit its two partials: at most c quads of 2 c - 1 rows
+// of four lanes (the field of view does not reach the grid's edge), 2 nx (nx - 1)
+// columns of the 2 nx^2.
+cudaError_t clear_shared(const hrrt_ctx *ctx, const float *samples, float *bc, int pairs, int frames) {
+  if (samples != bc) return cudaSuccess;
+  const size_t rows = (size_t)pairs * ctx->dg.samp_pair * 4, block = 2 * (size_t)ctx->npairs * ctx->vol;
+  return cudaMemset2DAsync(bc, block * sizeof(float), 0, rows * sizeof(float), frames, ctx->stream);
+}
+
 SubsetBufs ctx_bufs(hrrt_ctx *ctx) {
-  return SubsetBufs{ctx->d_image, ctx->q_prompts, ctx->q_add, ctx->d_ratio, ctx->d_bc, ctx->d_br, ctx->d_samples, one_frame()};
+  return SubsetBufs{ctx->d_image, ctx->q_prompts, ctx->q_add, ctx->d_ratio, ctx->d_bc, ctx->d_br, samples_of(ctx), one_frame()};
 }
 
 int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
@@ -230,6 +248,13 @@ int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
   const int *pv = ctx->d_pair_views + (size_t)s * ctx->npairs;
   float *nf = ctx->d_nfinv + (size_t)s * ctx->vol;
   const bool single = b.fr.n == 1 && !b.fr.map;
+  auto project = [&](const float *image) {
+    Launch L(ctx, "fp_kernel");
+    const cudaError_t e = launch_fp(g, image, b.samples, pv, 0, ctx->npairs, fw, ctx->fp_cnt[s], 1, b.prompts, b.add,
+                                    ctx->storage, b.ratio, ctx->quad_pair, b.fr, ctx->stream);
+    const cudaError_t c = clear_shared(ctx, b.samples, b.bc, ctx->npairs, b.fr.n);
+    return e != cudaSuccess ? e : c;
+  };
   const bool map = single && ctx->map_on && ctx->subsets_done >= ctx->map_first;
   if (single) ctx->subsets_done++;
   if (map) {
@@ -241,12 +266,7 @@ int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
       if (int rc = run_psf(ctx, b.image, ctx->d_image_psf)) return rc;
       proj = ctx->d_image_psf;
     }
-    {
-      Launch L(ctx, "fp_kernel");
-      CK(launch_fp(g, proj, b.samples, pv, 0, ctx->npairs, fw, ctx->fp_cnt[s], 1, b.prompts, b.add, ctx->storage, b.ratio, ctx->quad_pair,
-                   b.fr, ctx->stream),
-         "fp_kernel");
-    }
+    CK(project(proj), "fp_kernel");
     if (adj) {
       CK(launch_adj(g, b.ratio, ctx->quad_pair, bw, ctx->bp_cnt[s], b.bc, b.br, ctx->vol, b.fr, ctx->stream),
          "adj_kernel");
@@ -281,12 +301,7 @@ int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
     // correction image, then update
     if (b.fr.n != 1 || b.fr.map) return fail(ctx, HRRT_ERR_STATE, "PSF runs one frame at a time");
     if (int rc = run_psf(ctx, b.image, ctx->d_image_psf)) return rc;
-    {
-      Launch L(ctx, "fp_kernel");
-      CK(launch_fp(g, ctx->d_image_psf, b.samples, pv, 0, ctx->npairs, fw, ctx->fp_cnt[s], 1, b.prompts, b.add, ctx->storage, b.ratio,
-                   ctx->quad_pair, b.fr, ctx->stream),
-         "fp_kernel");
-    }
+    CK(project(ctx->d_image_psf), "fp_kernel");
     if (adj) {
       CK(launch_adj(g, b.ratio, ctx->quad_pair, bw, ctx->bp_cnt[s], b.bc, b.br, ctx->vol, b.fr, ctx->stream),
          "adj_kernel");
@@ -306,12 +321,7 @@ int run_subset(hrrt_ctx *ctx, int s, const SubsetBufs &b) {
     CK(launch_apply_corr(g, ctx->d_corr, b.image, nf, 0, ctx->stream), "update");
     return HRRT_OK;
   }
-  {
-    Launch L(ctx, "fp_kernel");
-    CK(launch_fp(g, b.image, b.samples, pv, 0, ctx->npairs, fw, ctx->fp_cnt[s], 1, b.prompts, b.add, ctx->storage, b.ratio, ctx->quad_pair,
-                 b.fr, ctx->stream),
-       "fp_kernel");
-  }
+  CK(project(b.image), "fp_kernel");
   if (adj) {
     {
       Launch L(ctx, "adj_kernel");
@@ -906,11 +916,10 @@ int hrrt_ctx_create(const hrrt_geom *gp, int device, hrrt_ctx **out) {
   ctx->d_image = dalloc<float>(ctx, ctx->vol, &e);
   ctx->d_nfinv = ctx->d_image ? dalloc<float>(ctx, (size_t)g.sp.subsets * ctx->vol, &e) : nullptr;
   ctx->d_ratio = ctx->d_nfinv ? dalloc<float>(ctx, (size_t)ctx->npairs * ctx->quad_pair, &e) : nullptr;
-  ctx->d_bc = ctx->d_ratio ? dalloc<float>(ctx, (size_t)ctx->npairs * ctx->vol, &e) : nullptr;
-  ctx->d_br = ctx->d_bc ? dalloc<float>(ctx, (size_t)ctx->npairs * ctx->vol, &e) : nullptr;
-  if (ctx->d_br) ctx->d_samples = dalloc<float>(ctx, (size_t)ctx->npairs * d.samp_pair * 4, &e);
+  ctx->d_bc = ctx->d_ratio ? dalloc<float>(ctx, 2 * (size_t)ctx->npairs * ctx->vol, &e) : nullptr;
+  if (ctx->d_bc) ctx->d_br = ctx->d_bc + (size_t)ctx->npairs * ctx->vol;
   const int pb = post_iteration_blocks(d);
-  ctx->d_partial = ctx->d_samples ? dalloc<double>(ctx, pb, &e) : nullptr;
+  ctx->d_partial = ctx->d_br ? dalloc<double>(ctx, pb, &e) : nullptr;
   ctx->d_sum = ctx->d_partial ? dalloc<double>(ctx, 1, &e) : nullptr;
   if (!ctx->d_sum) return bail(fail(ctx, HRRT_ERR_NOMEM, std::string("device allocation: ") + cudaGetErrorString(e)));
   // the adjoint runs with segment weights of 1 (its rows carry the forward
@@ -964,6 +973,7 @@ int hrrt_upload_inputs(hrrt_ctx *ctx, const int16_t *prompts, const float *rando
   if (storage < HRRT_STORE_F32 || storage > HRRT_STORE_F16) return fail(ctx, HRRT_ERR_ARG, "unknown storage");
   if (ctx->batch) return fail(ctx, HRRT_ERR_STATE, "the context serves a batch (hrrt_batch_destroy first)");
   if (int rc = ensure_input_buffers(ctx, storage)) return rc;
+  samples_of(ctx);
   if (int rc = upload_flat(ctx, prompts, randoms, norm, atten, scatter, storage, false, ctx->q_prompts, ctx->q_add,
                            ctx->q_mult))
     return rc;
@@ -1115,6 +1125,7 @@ int hrrt_reconstruct(hrrt_ctx *ctx, const int16_t *prompts, const float *randoms
     if (!ctx->pflat) return fail(ctx, HRRT_ERR_NOMEM, "reconstruct prompts");
     ctx->pflat_elems = pelems;
   }
+  samples_of(ctx);
   if (!ctx->copy_stream) {
     CK(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking), "copy stream");
     for (int b = 0; b < 2; b++) {
@@ -1317,8 +1328,10 @@ int hrrt_fp_pair(hrrt_ctx *ctx, const float *image_xyz, int view, float *prj) {
   CK(cudaMemcpyAsync(ctx->d_rows, prj, rows * 4, cudaMemcpyHostToDevice, ctx->stream), "fp_pair");
   {
     Launch L(ctx, "fp_kernel");
-    CK(launch_fp(ctx->dg, ctx->d_tmp_img, ctx->d_samples, nullptr, view, 1, dw, (int)work.size(), 0, nullptr, nullptr, 0, ctx->d_ratio, ctx->quad_pair, one_frame(), ctx->stream),
+    float *samples = ctx->d_samples ? ctx->d_samples : ctx->d_bc;
+    CK(launch_fp(ctx->dg, ctx->d_tmp_img, samples, nullptr, view, 1, dw, (int)work.size(), 0, nullptr, nullptr, 0, ctx->d_ratio, ctx->quad_pair, one_frame(), ctx->stream),
        "fp_kernel");
+    CK(clear_shared(ctx, samples, ctx->d_bc, 1, 1), "fp_pair");
   }
   CK(launch_quad_to_rows(ctx->dg, g.nbins, ctx->d_ratio, dw, (int)work.size(), ctx->d_rows, ctx->stream), "unpack");
   CK(cudaMemcpyAsync(prj, ctx->d_rows, rows * 4, cudaMemcpyDeviceToHost, ctx->stream), "fp_pair");
@@ -1333,7 +1346,7 @@ int hrrt_forward_project(hrrt_ctx *ctx, const float *image_xyz, float *sino) {
   if (!ctx->d_tmp_img) return fail(ctx, HRRT_ERR_NOMEM, "scratch");
   const size_t n = (size_t)g.segmentsize * g.nviews * g.nbins;
   float *dsino = nullptr;
-  e = cudaMalloc(&dsino, n * sizeof(float));
+  e = dmalloc(ctx, (void **)&dsino, n * sizeof(float));
   if (e != cudaSuccess) return fail(ctx, HRRT_ERR_NOMEM, "sinogram");
   QuadWork *dw = nullptr;
   auto done = [&](int rc) {
@@ -1357,19 +1370,22 @@ int hrrt_forward_project(hrrt_ctx *ctx, const float *image_xyz, float *sino) {
           work.push_back(QuadWork{(int16_t)k, (int16_t)x, (int16_t)(b + k), 0});
   }
   off.push_back((int)work.size());
-  if (e == cudaSuccess) e = cudaMalloc(&dw, work.size() * sizeof(QuadWork) + 16);
+  if (e == cudaSuccess) e = dmalloc(ctx, (void **)&dw, work.size() * sizeof(QuadWork) + 16);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(dw, work.data(), work.size() * sizeof(QuadWork), cudaMemcpyHostToDevice, ctx->stream);
+  float *samples = ctx->d_samples ? ctx->d_samples : ctx->d_bc;
   for (size_t b = 0; b + 1 < off.size() && e == cudaSuccess; b++) {
     const int cnt = off[b + 1] - off[b];
     {
       Launch L(ctx, "fp_kernel");
-      e = launch_fp(ctx->dg, ctx->d_tmp_img, ctx->d_samples, nullptr, (int)b * ctx->npairs,
+      e = launch_fp(ctx->dg, ctx->d_tmp_img, samples, nullptr, (int)b * ctx->npairs,
                     std::min(ctx->npairs, V2 - (int)b * ctx->npairs), dw + off[b], cnt, 0, nullptr, nullptr, 0, ctx->d_ratio, ctx->quad_pair, one_frame(), ctx->stream);
     }
     if (e == cudaSuccess)
       e = launch_quad_to_file(ctx->dg, g.nbins, ctx->d_ratio, ctx->quad_pair, dw + off[b], cnt, dsino, ctx->stream);
   }
+  const cudaError_t cleared = clear_shared(ctx, samples, ctx->d_bc, ctx->npairs, 1);
+  if (e == cudaSuccess) e = cleared;
   if (e == cudaSuccess) e = cudaMemcpyAsync(sino, dsino, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return done(cuda_fail(ctx, e, "forward_project"));
