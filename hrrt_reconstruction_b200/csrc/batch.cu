@@ -338,6 +338,9 @@ int hrrt_batch_create(hrrt_ctx *ctx, int nframes, int storage, const float *norm
   if (b->bc) b->br = b->bc + (size_t)ctx->npairs * ctx->vol;
   b->partial = b->br ? b->alloc<double>((size_t)b->group * b->pb, &e) : nullptr;
   if (!b->partial) return bail(fail(ctx, HRRT_ERR_NOMEM, "batch: scratch"));
+  // the columns beside the field of view stay as they are here
+  e = cudaMemsetAsync(b->bc, 0, (size_t)b->group * 2 * ctx->npairs * ctx->vol * sizeof(float), ctx->stream);
+  if (e != cudaSuccess) return bail(cuda_fail(ctx, e, "batch: scratch"));
   b->samples = b->alloc<float>((size_t)b->group * samp, &e);
   if (!b->samples) b->samples = b->bc;
   ctx->batch = b;
