@@ -225,8 +225,9 @@ __device__ __forceinline__ SamplePt sample_point(int a, int b, int c, int N, int
 //                      outputs, row by row in the reference's order.
 // Samples of a quad, entries of 4 lanes: [zp] centre column, then per row
 // y = cyl0[x] .. c-1 [2 halves][zp], at g.samp_off[x] of its pair slot.
-// fp_kernel is bound by shared memory (L1 87 % busy at span 3: 2 x 8 bytes for
-// 6 packed operations), fp_sample_kernel by the latency of its L2 reads.
+// fp_kernel is bound by shared memory (L1 92 % busy at span 3: 2 x 8 bytes for
+// 6 packed operations), fp_sample_kernel by L1 (76 % busy) and the latency of
+// its L2 reads.
 // Measured on B200, us a subset: span 3 1892 -> 1037 + 241, span 9 860 -> 475
 // + 241, a 24-ring scanner 53 -> 26 + 6; before, one kernel sampled with four
 // warps (bulk tensor copies of the corner columns) beside 28 warps of 9-plane
@@ -552,18 +553,18 @@ __global__ void __launch_bounds__(kFpMaxWarps * 32, 1) fp_kernel(DevGeom g, cons
 // one from the ray of view p+nviews/2 (its row quad); they go to Bc and Br and
 // are added in the rotate-back, which is the reference's assign-then-
 // accumulate order.
-// What bounds it is instruction issue and the latency that 16 warps leave
-// uncovered: per (row group, side of a
-// group) a thread reads 6 shared planes for 16 outputs -- adjacent rows read
-// the segment less than a plane apart, so four rows share a window -- and
-// issues 64 packed FMAs and about as many other instructions.  One row and 8
-// planes a thread (9 shared planes for 8 outputs, an address each) took
-// 1.384 ms a span-3 subset and 0.509 ms a span-9 one; this 0.996 and 0.381,
-// to the same bits.  Measured and not used: one plane for all rows and
-// differences (bp_rows: 0.892 and 0.343 ms; loses sparse data's accuracy), and
-// in that form the row pattern as arithmetic instead of a branch (1.021 ms),
-// lane pairs split over two threads for twice the warps (0.941 ms), no prefetch
-// of the next entry (0.977 ms).
+// What bounds it is instruction issue and the latency that 16 warps an SM leave
+// uncovered (issue 55 %, FMA pipe 48 %, L1 45 % busy at span 3): per (row
+// group, side of a group) a thread reads 6 shared planes for 16 outputs --
+// adjacent rows read the segment less than a plane apart, so four rows share a
+// window -- and issues 64 packed FMAs and about as many other instructions.
+// One row and 8 planes a thread (9 shared planes for 8 outputs, an address
+// each) took 1.384 ms a span-3 subset and 0.509 ms a span-9 one; this 0.990
+// and 0.375, to the same bits (one pair with ACC: 385 us and 154).  Measured
+// and not used: one plane for all rows and differences (bp_rows: 0.892 and
+// 0.343 ms; loses sparse data's accuracy), and in that form the row pattern as
+// arithmetic instead of a branch (1.021 ms), lane pairs split over two threads
+// for twice the warps (0.941 ms), no prefetch of the next entry (0.977 ms).
 // ============================================================================
 // The shared planes are stored by phase, plane i at slot bp_slot(i): eight
 // lanes of a warp take consecutive 4-plane runs of one row group, so that
@@ -1471,10 +1472,10 @@ __global__ void scale_pairs_kernel(DevGeom g, const T *__restrict__ src, const i
 // Launches a kernel that has `ctas` CTAs resident per SM by its registers; what
 // their shared memory leaves of the SM's stays L1, which holds the sampling
 // tables the projectors read (the whole SM's memory as shared memory instead:
-// adjoint 1200 us a subset at span 9 against 1057, back projector 361 against
-// 343).  The split goes with the launch, and the limit that belongs to the
-// kernel itself is always the same: contexts of other sizes may launch it from
-// other threads.
+// adjoint 1200 us a subset at span 9 against 1057, the back projector of that
+// build 361 against 343).  The split goes with the launch, and the limit that
+// belongs to the kernel itself is always the same: contexts of other sizes may
+// launch it from other threads.
 template <typename... P, typename... A>
 cudaError_t launch_smem(void (*k)(P...), long long grid, int threads, size_t smem, int ctas, cudaStream_t st,
                         A... args) {
@@ -1535,7 +1536,7 @@ cudaError_t launch_fp(const DevGeom &g, const float *image, float *samples, cons
     FrameStrides part = fr;
     part.n = std::min(per, fr.n - f0);
     if (fr.map) part.map = fr.map + f0;
-    // 8 rows a warp, fewer where that leaves SMs without their two CTAs
+    // 16 rows a warp, fewer where that leaves less than eight CTAs an SM
     const int nx = (g.c + T - 1) / T, nz = 2 * npairs * part.n;
     int steps = 16;
     while (steps > 1 && (long long)nx * nz * (g.c / (T * steps) + 1) < 8 * 148) steps /= 2;

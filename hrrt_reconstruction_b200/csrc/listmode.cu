@@ -58,8 +58,8 @@ constexpr int kSinoPlane = 256 * 288;
 // the end.  Partitioned: events scattered by 64 MB partition and added
 // partition by partition in L2.  On B200, for 1e8 / 4e8 events: direct 4.8 /
 // 18.9 ms (the random read-modify-write of a DRAM sector per event bounds it),
-// wide 7.0 / 21.7 (the same, and a clear and a fold of 4-byte counters),
-// partitioned 5.4 / 20.0 (two parses more), so the other two run only when
+// wide 7.1 / 22.1 (the same, and a clear and a fold of 4-byte counters),
+// partitioned 5.5 / 19.9 (two parses more), so the other two run only when
 // asked for.  A fourth way, rebinning every event into a 4-byte record in
 // stream order and adding the records in a separate pass with 30 registers a
 // thread (eight blocks per SM, more adds in flight), was slower as well: the
