@@ -1692,6 +1692,8 @@ int hrrt_rotate_add(hrrt_ctx *ctx, const float *imagebuf_xyz, int view, float *c
     CK(launch_rotback(ctx->dg, dv, 1, ctx->d_bc, nullptr, ctx->vol, nullptr, nullptr, ctx->d_tmp_img, 2, one_frame(), ctx->stream),
        "rotback");
   }
+  // the partials stay zero beside the field of view, which the image need not be
+  CK(cudaMemsetAsync(ctx->d_bc, 0, ctx->vol * 4, ctx->stream), "rotate");
   CK(cudaMemcpyAsync(corr_xyz, ctx->d_tmp_img, ctx->vol * 4, cudaMemcpyDeviceToHost, ctx->stream), "rotate");
   CK(cudaStreamSynchronize(ctx->stream), "rotate");
   return HRRT_OK;
